@@ -69,7 +69,7 @@ typedef struct {
     double tol;          /* relative residual target ||b-Ax||/||b|| (default 1e-8) */
     int max_iter;        /* outer iteration cap (default 200) */
     int precision;       /* 0: FP32 V-cycle in an FP64 outer loop; 1: FP64 V-cycle */
-    int restart;         /* GCR restart length (default 16, at most 18) */
+    int restart;         /* GMRES restart length (default 16, at most 18) */
     double omega;        /* cell-block smoother damping (default 0.7) */
     int use_graphs;      /* capture the V-cycle in a CUDA graph (default 1) */
     int smoother;        /* cell-block smoother: 1 = exact 7x7 cell solve with the cell
@@ -83,7 +83,7 @@ typedef struct {
 } p2_params;
 
 typedef struct {
-    int iterations;          /* outer (GCR) iterations */
+    int iterations;          /* outer (GMRES) iterations */
     double rel_residual;     /* final ||b-Ax||/||b|| of the level-0 system, FP64 */
     double rel_residual0;    /* initial */
     double ms_total;         /* device time of the whole solve (CUDA events) */
@@ -103,7 +103,7 @@ typedef struct {
     int trial_iters;     /* outer iterations per trial */
     int sweep_max;       /* most sweeps on any level: sweeps on level l >= 1 =
                             min(sweep_max, npre[0] * sweep_growth^l) with the configured npre[0] */
-    int restart;         /* chosen GCR restart length (12 or the configured one, whichever
+    int restart;         /* chosen GMRES restart length (12 or the configured one, whichever
                             full solve of the chosen schedule was faster) */
     int sweeps0;         /* pre- (and post-) sweeps on level 0: npre[0], or half of it */
 } p2_tune_info;
@@ -158,7 +158,7 @@ p2_status p2_get_solution(p2_ctx *ctx, double *vx, double *vy, double *vz, doubl
  * or diagonal cell block, constant or doubling sweeps per coarser level, the
  * configured or half the sweeps on level 0), estimates each candidate's time
  * to p2_params.tol from its measured rate and time per iteration, keeps the
- * cheapest in this context's parameters, then picks the GCR restart length
+ * cheapest in this context's parameters, then picks the GMRES restart length
  * (12 or the configured one) by two full solves.  Call it once per model
  * before the time loop. */
 p2_status p2_autotune(p2_ctx *ctx, int trial_iters, p2_tune_info *info);

@@ -337,7 +337,7 @@ struct Vec4 {
 
 
 // Per-axis transfer tables (built on the host from the reference's index
-// rules) and reduction job descriptors, shared by the kernels and the host.
+// rules), shared by the kernels and the host.
 constexpr int kRedBlocks = 592;  // 4 x 148 SMs
 struct AxisMap {
     const int *lo;
@@ -351,18 +351,4 @@ struct TransferView {
     AxisMap m[3][3];  // [axis][type]
 };
 
-struct DotJob {
-    const double *a[4];
-    const double *b[4];
-};
-constexpr int kMaxDots = 20;
-struct DotJobs {
-    DotJob j[kMaxDots];
-    int nd;
-};
-
-struct VecList {
-    const double *v[kMaxDots][4];
-    int nv;
-};
 }  // namespace p2

@@ -1022,8 +1022,7 @@ __global__ void k_bc_consts(int nbc, const int *bu, const float *bconst, Vec4<T>
 }
 
 // ---------------------------------------------------------------------------
-// Deterministic reductions: fixed grid, grid-stride, block tree, then one
-// block sums the partials in order.
+// Deterministic reductions: a block tree; partials are summed in block order.
 
 __device__ __forceinline__ double block_sum(double v, double *sh)
 {
@@ -1038,69 +1037,6 @@ __device__ __forceinline__ double block_sum(double v, double *sh)
     }
     __syncthreads();
     return s;
-}
-
-// nd dot products of 4-field vectors: out[q] = sum a_q . b_q (pairs given by
-// pointer tables), skipping the pinned pressure cell when skip_node >= 0.
-// One sweep over the nodes for all pairs: a vector shared by several pairs
-// (the new direction against every stored one) comes from DRAM once and is
-// re-read from L1.
-// ND, the number of pairs, is a template parameter: the accumulators stay in
-// registers whatever ND is, and the node loop is unrolled so that each thread
-// has several independent loads in flight (one load at a time per thread left
-// the sweep latency-bound at a fraction of the HBM bandwidth).
-template <int ND>
-__global__ void k_dots_partial(DotJobs jobs, int n, int skip_node, double *partial)
-{
-    __shared__ double sh[32];
-    double s[ND];
-#pragma unroll
-    for (int q = 0; q < ND; q++) s[q] = 0;
-    const int stride = gridDim.x * blockDim.x;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const double *a[ND], *b[ND];
-#pragma unroll
-        for (int q = 0; q < ND; q++) { a[q] = jobs.j[q].a[c]; b[q] = jobs.j[q].b[c]; }
-#pragma unroll 4
-        for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += stride) {
-            if (c == 0 && u == skip_node) continue;
-#pragma unroll
-            for (int q = 0; q < ND; q++) s[q] += __ldg(a[q] + u) * __ldg(b[q] + u);
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < ND; q++) {
-        const double t = block_sum(s[q], sh);
-        if (threadIdx.x == 0) partial[q * gridDim.x + blockIdx.x] = t;
-    }
-}
-
-// k_dots_partial<jobs.nd> on kRedBlocks blocks of kThreads threads
-inline cudaError_t launch_dots(cudaStream_t st, const DotJobs &jobs, int n, int skip_node, double *partial)
-{
-    switch (jobs.nd) {
-#define P2_DOTS_CASE(N) \
-    case N: k_dots_partial<N><<<kRedBlocks, kThreads, 0, st>>>(jobs, n, skip_node, partial); break;
-        P2_DOTS_CASE(1) P2_DOTS_CASE(2) P2_DOTS_CASE(3) P2_DOTS_CASE(4) P2_DOTS_CASE(5) P2_DOTS_CASE(6)
-        P2_DOTS_CASE(7) P2_DOTS_CASE(8) P2_DOTS_CASE(9) P2_DOTS_CASE(10) P2_DOTS_CASE(11) P2_DOTS_CASE(12)
-        P2_DOTS_CASE(13) P2_DOTS_CASE(14) P2_DOTS_CASE(15) P2_DOTS_CASE(16) P2_DOTS_CASE(17) P2_DOTS_CASE(18)
-        P2_DOTS_CASE(19) P2_DOTS_CASE(20)
-#undef P2_DOTS_CASE
-    default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
-__global__ void k_dots_final(int nd, int nparts, const double *partial, double *out)
-{
-    __shared__ double sh[32];
-    for (int q = 0; q < nd; q++) {
-        double s = 0;
-        for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += partial[q * nparts + i];
-        double t = block_sum(s, sh);
-        if (threadIdx.x == 0) out[q] = t;
-    }
 }
 
 // Sum of volume * b_P over continuity rows and of the volumes (compatibility).
@@ -1121,98 +1057,6 @@ __global__ void k_compat_apply(LevelView<T> L, T *bp, const double *sums)
 
 // ---------------------------------------------------------------------------
 // Small vector kernels.
-__global__ void k_axpy4(int n, const double *alpha, double sign, Vec4<double> y, Vec4<double> x)
-{
-    int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= n) return;
-    double a = sign * alpha[0];
-#pragma unroll
-    for (int c = 0; c < 4; c++) y.c[c][u] += a * x.c[c][u];
-}
-
-// GCR scalars kept on the device (no host round trip inside an iteration):
-// coef[j] = (q, Q_j) / (Q_j, Q_j) for the k stored directions.
-__global__ void k_gcr_coef(int k, const double *dots, const double *qq, double *coef)
-{
-    const int j = threadIdx.x;
-    if (j < k) coef[j] = dots[j] / qq[j];
-}
-// qq_k = (q', q') and alpha = (r, q') / qq_k from dots[0], dots[1]; a
-// direction without a positive norm sets flag[0] = 1 and alpha = 0.
-__global__ void k_gcr_alpha(const double *dots, double *qqk, double *alpha, double *flag)
-{
-    if (threadIdx.x != 0) return;
-    const double qq = dots[0];
-    qqk[0] = qq;
-    if (qq > 0) {
-        alpha[0] = dots[1] / qq;
-    } else {
-        alpha[0] = 0;
-        flag[0] = 1;
-    }
-}
-
-// Classical Gram-Schmidt update of the new direction with its dot products:
-//   q' = q - sum_j coef_j Q_j (in place), z' = z - sum_j coef_j Z_j (z read
-//   from zs, stored as S; z' written to zo, which may be zs),
-// and per block the partial sums of (q', q') and (r, q'), in the node loop
-// of k_dots_partial (kRedBlocks blocks of kThreads threads, components outer,
-// nodes strided, the pinned pressure cell skipped), so the sums are the ones
-// a separate dot-product pass over q' would give.  NV, the number of stored
-// directions, is a template parameter: the coefficients stay in registers and
-// the loads of all directions of a node are issued together.
-template <int NV, typename S>
-__global__ void k_cgs_update_dots(int n, const double *coef, Vec4<double> q, VecList X, Vec4<S> zs,
-                                  Vec4<double> zo, VecList Z, Vec4<double> r, int skip_node, double *partial)
-{
-    __shared__ double sh[32];
-    double cf[NV > 0 ? NV : 1];
-#pragma unroll
-    for (int j = 0; j < NV; j++) cf[j] = coef[j];
-    double sqq = 0, srq = 0;
-    const int stride = gridDim.x * blockDim.x;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += stride) {
-            double sy = q.c[c][u], sz = (double)zs.c[c][u];
-#pragma unroll
-            for (int j = 0; j < NV; j++) {
-                sy -= cf[j] * X.v[j][c][u];
-                sz -= cf[j] * Z.v[j][c][u];
-            }
-            q.c[c][u] = sy;
-            zo.c[c][u] = sz;
-            if (c == 0 && u == skip_node) continue;
-            sqq += sy * sy;
-            srq += r.c[c][u] * sy;
-        }
-    }
-    const double t0 = block_sum(sqq, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = t0;
-    const double t1 = block_sum(srq, sh);
-    if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = t1;
-}
-
-// k_cgs_update_dots<nv, S> on kRedBlocks blocks of kThreads threads
-template <typename S>
-inline cudaError_t launch_cgs_update_dots(cudaStream_t st, int nv, int n, const double *coef, const Vec4<double> &q,
-                                          const VecList &X, const Vec4<S> &zs, const Vec4<double> &zo,
-                                          const VecList &Z, const Vec4<double> &r, int skip_node, double *partial)
-{
-    switch (nv) {
-#define P2_CGS_CASE(N)                                                                                          \
-    case N:                                                                                                     \
-        k_cgs_update_dots<N, S><<<kRedBlocks, kThreads, 0, st>>>(n, coef, q, X, zs, zo, Z, r, skip_node, partial); \
-        break;
-        P2_CGS_CASE(0) P2_CGS_CASE(1) P2_CGS_CASE(2) P2_CGS_CASE(3) P2_CGS_CASE(4) P2_CGS_CASE(5) P2_CGS_CASE(6)
-        P2_CGS_CASE(7) P2_CGS_CASE(8) P2_CGS_CASE(9) P2_CGS_CASE(10) P2_CGS_CASE(11) P2_CGS_CASE(12)
-        P2_CGS_CASE(13) P2_CGS_CASE(14) P2_CGS_CASE(15) P2_CGS_CASE(16) P2_CGS_CASE(17)
-#undef P2_CGS_CASE
-    default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
 __global__ void k_f32_to_f64(int n, Vec4<float> a, Vec4<double> b)
 {
     int u = blockIdx.x * blockDim.x + threadIdx.x;

@@ -2,9 +2,10 @@
 // transfer tables, the V-cycle (FP32 or FP64) and the FP64 outer loop.
 //
 // Solve structure (move3mgNew.c:1791 vpiterate is the reference entry point):
-//   outer FP64 GCR on the level-0 system, each iteration: true residual
-//   r = b - A x in FP64, z = V(r) one V-cycle (FP32 in mixed mode), q = A z,
-//   Gram-Schmidt against the previous directions, x += alpha z.
+//   outer FP64 flexible GMRES on the level-0 system, each iteration: one
+//   V-cycle z = V(w) (FP32 in mixed mode), q = A z in FP64, Gram-Schmidt
+//   against the basis; per restart and before the solve returns x += sum y z
+//   and the true residual r = b - A x in FP64.
 //   V-cycle: on levels 0..L-1 cell-block smoothing + residual + restriction
 //   (vprestrict), dense inverse on the coarsest level (replaces PARDISO),
 //   prolongation (vpprolong) + smoothing back up.
@@ -21,6 +22,7 @@
 #include <vector>
 
 #include "p2_kernels.cuh"
+#include "p2_krylov.cuh"
 #include "p2_solver.h"
 #include "p2_sweep.cuh"
 #include "p2_zmarch.cuh"
@@ -595,7 +597,7 @@ void Solver::allocate_work()
     f0.nxz = (float *)arena.alloc(sizeof(float) * n0);
     f0.nyz = (float *)arena.alloc(sizeof(float) * n0);
     // outer loop vectors
-    int m = std::max(1, std::min(prm.restart, kMaxDots - 2));
+    int m = std::max(1, std::min(prm.restart, kMaxBasis - 1));
     restart = m;
     auto v64n = [&](Vec4<double> &v) {
         double *p = (double *)arena.alloc(sizeof(double) * 4 * n0);
@@ -604,11 +606,26 @@ void Solver::allocate_work()
     };
     v64n(gx); v64n(gb); v64n(gr);
     if (prm.precision == 1) L[0].b64 = gr;  // the FP64 cycle's level-0 right-hand side is the residual
-    qq_dev = (double *)arena.alloc(sizeof(double) * m);
-    Z.assign(m, Vec4<double>());
-    Q.assign(m, Vec4<double>());
-    for (int q = 0; q < m; q++) { v64n(Z[q]); v64n(Q[q]); }
-    partial = (double *)arena.alloc(sizeof(double) * kRedBlocks * kMaxDots);
+    W.assign(m + 1, Vec4<double>());
+    for (auto &v : W) v64n(v);
+    Z32.clear();
+    Z64.clear();
+    for (int q = 0; q < m; q++) {
+        if (prm.precision == 0) {
+            float *p = (float *)arena.alloc(sizeof(float) * 4 * n0);
+            Vec4<float> v;
+            for (int c = 0; c < 4; c++) v.c[c] = p + c * n0;
+            v.n = (int)n0;
+            Z32.push_back(v);
+        } else {
+            Z64.emplace_back();
+            v64n(Z64.back());
+        }
+    }
+    ww = (double *)arena.alloc(sizeof(double) * (m + 1));
+    hcol = (double *)arena.alloc(sizeof(double) * HC_LEN);
+    partial = (double *)arena.alloc(sizeof(double) * kRedBlocks * kMaxBasis);
+    dticket = (unsigned *)arena.alloc(sizeof(unsigned) * 4);
     {
         long maxc = 1;
         for (int l = 1; l < nl; l++) maxc = std::max<long>(maxc, L[l].n);
@@ -628,9 +645,8 @@ void Solver::allocate_work()
             Lv.compat_vol = vt;
         }
     }
-    dots = (double *)arena.alloc(sizeof(double) * kMaxDots * 2);
-    scal = (double *)arena.alloc(sizeof(double) * 64);  // [0,1] compat sums, [2] alpha, [3] shift, [8..] GS coefficients
-    P2_CUDA_TRY(cudaMallocHost(&hdots_raw, sizeof(double) * kMaxDots * 2));
+    scal = (double *)arena.alloc(sizeof(double) * 8);  // [0,1] compat sums, [3] pressure shift
+    P2_CUDA_TRY(cudaMallocHost(&hdots_raw, sizeof(double) * HC_LEN));
     hdots.reset(hdots_raw, [](double *p) { cudaFreeHost(p); });
     // coarse free-unknown set
     build_coarse_index();
@@ -1135,19 +1151,14 @@ void Solver::upload_nodes(const float *nu, const float *ro, const float *nxx, co
     nodes_ready = true;
 }
 
-void Solver::dots_sync(const DotJobs &jobs)
+// ||W_0||^2 (also kept in ww[0]); waits for the stream
+double Solver::residual_norm2()
 {
-    P2_CUDA_TRY(launch_dots(st, jobs, L[0].n, L[0].pin, partial)); P2_COUNT_LAUNCH();
-    k_dots_final<<<1, 1024, 0, st>>>(jobs.nd, kRedBlocks, partial, dots); P2_COUNT_LAUNCH();
-    P2_CUDA_TRY(cudaMemcpyAsync(hdots.get(), dots, sizeof(double) * jobs.nd, cudaMemcpyDeviceToHost, st));
+    P2_CUDA_TRY(launch_basis_dots(st, 0, 2L * L[0].n, W[0].c[0], Basis{}, L[0].pin, partial, dticket, ww, hcol));
+    P2_COUNT_LAUNCH();
+    P2_CUDA_TRY(cudaMemcpyAsync(hdots.get(), hcol + HC_QQ, sizeof(double), cudaMemcpyDeviceToHost, st));
     P2_CUDA_TRY(cudaStreamSynchronize(st));
-}
-
-static DotJob job(const Vec4<double> &a, const Vec4<double> &b)
-{
-    DotJob j;
-    for (int c = 0; c < 4; c++) { j.a[c] = a.c[c]; j.b[c] = b.c[c]; }
-    return j;
+    return hdots.get()[0];
 }
 
 // out = b - A x (mode 0) or A x (mode 1) on level 0 in FP64 (x stored as
@@ -1166,11 +1177,9 @@ void Solver::rows0(const Vec4<S> &x, Vec4<double> &out, Vec4<float> *r32, int mo
     }
 }
 
-// One preconditioning V-cycle from zero for the level-0 right-hand side r:
-// the mixed cycle reads float(r), which the true residual wrote into b32;
-// the FP64 cycle's level-0 right-hand side is r itself (b64 of level 0 is
-// gr).  The correction stays in x32 / x64; the Gram-Schmidt update reads it
-// from there.
+// One preconditioning V-cycle from zero for the level-0 right-hand side b32 /
+// b64 (the copy of the current basis vector in the cycle's type).  The
+// correction stays in x32 / x64.
 void Solver::precondition()
 {
     Level &L0 = L[0];
@@ -1240,81 +1249,118 @@ p2_solve_info Solver::solve()
                      graphs[prm.precision == 0 ? 0 : 1].kernels);
     }
     // b-norm of the pinned system: every row but the pin cell's, plus the pin value
-    DotJobs J{};
-    J.j[0] = job(gb, gb);
-    J.nd = 1;
-    dots_sync(J);
-    double bnorm2 = hdots.get()[0] + (L0.pin >= 0 ? L0.pinval * L0.pinval : 0.0);
+    const bool f32 = prm.precision == 0;
+    const long n2 = 2L * n;
+    const size_t vec64 = sizeof(double) * 4 * n;
+    P2_CUDA_TRY(cudaMemcpyAsync(W[0].c[0], gb.c[0], vec64, cudaMemcpyDeviceToDevice, st));
+    double bnorm2 = residual_norm2() + (L0.pin >= 0 ? L0.pinval * L0.pinval : 0.0);
     double bnorm = std::sqrt(bnorm2);
     if (!(bnorm > 0)) bnorm = 1.0;
-    int m = restart, k = 0, it = 0;
+    const int m = restart;
+    int it = 0;
     float vc_ms = 0;
     double rel = 0;
-    if ((int)vc_ev.size() < 2) {
-        vc_ev.resize(2);
-        for (auto &e : vc_ev) P2_CUDA_TRY(cudaEventCreate(&e));
-    }
     std::vector<std::pair<int, int>> vc_marks;  // event pairs around each V-cycle
-    P2_CUDA_TRY(cudaMemsetAsync(scal + 4, 0, sizeof(double), st));  // non-positive direction norm flag
+    Basis B{};
+    for (int j = 0; j <= m; j++) B.v[j] = (const double2 *)W[j].c[0];
+    // Flexible GMRES(m): A Z = W H with W orthogonal and not normalised, norms
+    // nrm_j; H's columns scaled by the norms, reduced by Givens rotations on the
+    // host as they arrive.  Its iterates are those of GCR(m) on the same
+    // corrections, but only one basis is orthogonalised and the solution and the
+    // true residual are formed once per restart: 2 k + 6 level-0 vectors per
+    // iteration with k stored ones where GCR moved 5 k + 12 and the residual rows.
+    // At 257^3 the outer loop went from 6.27 to 3.54 ms per iteration (V-cycle 12.8).
+    std::vector<double> R((size_t)m * m), cs(m), sn(m), g(m + 1), nrm(m + 1), y(m);
     for (;;) {
-        // true FP64 residual (its float copy is the mixed cycle's right-hand side)
-        rows0(gx, gr, prm.precision == 0 ? &L0.b32 : nullptr, 0);
-        // the one host synchronisation of an iteration: the residual norm and
-        // the flag of the previous iteration's direction
-        J.nd = 1;
-        J.j[0] = job(gr, gr);
-        P2_CUDA_TRY(launch_dots(st, J, L0.n, L0.pin, partial)); P2_COUNT_LAUNCH();
-        k_dots_final<<<1, 1024, 0, st>>>(1, kRedBlocks, partial, dots); P2_COUNT_LAUNCH();
-        P2_CUDA_TRY(cudaMemcpyAsync(hdots.get(), dots, sizeof(double), cudaMemcpyDeviceToHost, st));
-        P2_CUDA_TRY(cudaMemcpyAsync(hdots.get() + 1, scal + 4, sizeof(double), cudaMemcpyDeviceToHost, st));
-        P2_CUDA_TRY(cudaStreamSynchronize(st));
-        double rr = hdots.get()[0];
+        // true FP64 residual, with its copy for the V-cycle
+        rows0(gx, W[0], f32 ? &L0.b32 : nullptr, 0);
+        if (!f32) P2_CUDA_TRY(cudaMemcpyAsync(L0.b64.c[0], W[0].c[0], vec64, cudaMemcpyDeviceToDevice, st));
+        const double rr = residual_norm2();
         rel = std::sqrt(rr) / bnorm;
         if (it == 0) info.rel_residual0 = rel;
         if (verbose) std::fprintf(stderr, "p2cuda: iteration %d rel residual %.3e\n", it, rel);
-        if (hdots.get()[1] != 0.0 || !std::isfinite(rel)) { info.status = P2_ERR_NAN; break; }
+        if (!std::isfinite(rel)) { info.status = P2_ERR_NAN; break; }
         if (rel <= prm.tol) { info.status = P2_OK; break; }
         if (it >= prm.max_iter) { info.status = P2_ERR_NOT_CONVERGED; break; }
-        Vec4<double> &z = Z[k], &q = Q[k];
-        if (it >= lu_overlap_iters) lu_finish();
-        coarse_mode = lu_pending ? 1 : 0;
-        const int e0 = 2 * (int)vc_marks.size();
-        if ((int)vc_ev.size() < e0 + 2) {
-            const size_t old = vc_ev.size();
-            vc_ev.resize(e0 + 2);
-            for (size_t e = old; e < vc_ev.size(); e++) P2_CUDA_TRY(cudaEventCreate(&vc_ev[e]));
+        nrm[0] = g[0] = std::sqrt(rr);
+        int k = 0;
+        bool bad = false;
+        while (k < m && it < prm.max_iter) {
+            if (it >= lu_overlap_iters) lu_finish();
+            coarse_mode = lu_pending ? 1 : 0;
+            const int e0 = 2 * (int)vc_marks.size();
+            while ((int)vc_ev.size() < e0 + 2) {
+                cudaEvent_t e = nullptr;
+                P2_CUDA_TRY(cudaEventCreate(&e));
+                vc_ev.push_back(e);
+            }
+            P2_CUDA_TRY(cudaEventRecord(vc_ev[e0], st));
+            precondition();
+            P2_CUDA_TRY(cudaEventRecord(vc_ev[e0 + 1], st));
+            vc_marks.push_back({e0, e0 + 1});
+            // Z_k = the correction, W_{k+1} = A Z_k, orthogonalised
+            Vec4<double> &q = W[k + 1];
+            if (f32) {
+                P2_CUDA_TRY(cudaMemcpyAsync(Z32[k].c[0], L0.x32.c[0], vec64 / 2, cudaMemcpyDeviceToDevice, st));
+                rows0(L0.x32, q, nullptr, 1);
+            } else {
+                P2_CUDA_TRY(cudaMemcpyAsync(Z64[k].c[0], L0.x64.c[0], vec64, cudaMemcpyDeviceToDevice, st));
+                rows0(L0.x64, q, nullptr, 1);
+            }
+            P2_CUDA_TRY(launch_basis_dots(st, k + 1, n2, q.c[0], B, L0.pin, partial, dticket, ww, hcol)); P2_COUNT_LAUNCH();
+            if (f32)
+                P2_CUDA_TRY(launch_basis_update<float2>(st, k + 1, n2, q.c[0], B, L0.b32.c[0], L0.pin, partial, dticket,
+                                                        ww, hcol));
+            else
+                P2_CUDA_TRY(launch_basis_update<double2>(st, k + 1, n2, q.c[0], B, L0.b64.c[0], L0.pin, partial,
+                                                         dticket, ww, hcol));
+            P2_COUNT_LAUNCH();
+            // the one host synchronisation of an iteration
+            double *hc = hdots.get();
+            P2_CUDA_TRY(cudaMemcpyAsync(hc, hcol, sizeof(double) * HC_LEN, cudaMemcpyDeviceToHost, st));
+            P2_CUDA_TRY(cudaStreamSynchronize(st));
+            it++;
+            const double sigma = hc[HC_SIGMA], wn2 = hc[HC_WW];
+            // a direction without a positive norm, or not a number
+            if (!(hc[HC_QQ] > 0) || !std::isfinite(wn2) || !std::isfinite(hc[HC_QQ])) { bad = true; break; }
+            nrm[k + 1] = std::sqrt(wn2);
+            double *col = &R[(size_t)k * m];
+            for (int j = 0; j <= k; j++) col[j] = hc[j] * nrm[j];
+            double sub = nrm[k + 1] / sigma;
+            for (int j = 0; j < k; j++) {
+                const double t = cs[j] * col[j] + sn[j] * col[j + 1];
+                col[j + 1] = -sn[j] * col[j] + cs[j] * col[j + 1];
+                col[j] = t;
+            }
+            const double d = std::hypot(col[k], sub);
+            cs[k] = col[k] / d;
+            sn[k] = sub / d;
+            col[k] = d;
+            g[k + 1] = -sn[k] * g[k];
+            g[k] *= cs[k];
+            k++;
+            rel = std::fabs(g[k]) / bnorm;
+            if (verbose) std::fprintf(stderr, "p2cuda: iteration %d rel residual %.3e (estimate)\n", it, rel);
+            if (rel <= prm.tol || !(wn2 > 0)) break;
         }
-        P2_CUDA_TRY(cudaEventRecord(vc_ev[e0], st));
-        precondition();
-        P2_CUDA_TRY(cudaEventRecord(vc_ev[e0 + 1], st));
-        vc_marks.push_back({e0, e0 + 1});
-        // q = A c for the correction c (x32 or x64 of level 0)
-        if (prm.precision == 0) rows0(L0.x32, q, nullptr, 1);
-        else rows0(L0.x64, q, nullptr, 1);
-        // classical Gram-Schmidt against the stored directions: coefficients
-        // on the device, then one pass that updates q and z and sums (q', q')
-        // and (r, q'), then alpha on the device and the solution update
-        if (k > 0) {
-            J.nd = 0;
-            for (int j = 0; j < k; j++) J.j[J.nd++] = job(q, Q[j]);
-            P2_CUDA_TRY(launch_dots(st, J, L0.n, L0.pin, partial)); P2_COUNT_LAUNCH();
-            k_dots_final<<<1, 1024, 0, st>>>(k, kRedBlocks, partial, dots); P2_COUNT_LAUNCH();
-            k_gcr_coef<<<1, 32, 0, st>>>(k, dots, qq_dev, scal + 8); P2_COUNT_LAUNCH();
+        if (bad) { info.status = P2_ERR_NAN; break; }
+        // x += sum y_j Z_j, y = R^-1 g
+        for (int i = k - 1; i >= 0; i--) {
+            double s = g[i];
+            for (int j = i + 1; j < k; j++) s -= R[(size_t)j * m + i] * y[j];
+            y[i] = s / R[(size_t)i * m + i];
         }
-        VecList X{}, Zl{};
-        for (int j = 0; j < k; j++)
-            for (int c = 0; c < 4; c++) { X.v[j][c] = Q[j].c[c]; Zl.v[j][c] = Z[j].c[c]; }
-        X.nv = Zl.nv = k;
-        if (prm.precision == 0)
-            P2_CUDA_TRY(launch_cgs_update_dots<float>(st, k, (int)n, scal + 8, q, X, L0.x32, z, Zl, gr, L0.pin, partial));
-        else
-            P2_CUDA_TRY(launch_cgs_update_dots<double>(st, k, (int)n, scal + 8, q, X, L0.x64, z, Zl, gr, L0.pin, partial));
-        P2_COUNT_LAUNCH();
-        k_dots_final<<<1, 1024, 0, st>>>(2, kRedBlocks, partial, dots); P2_COUNT_LAUNCH();
-        k_gcr_alpha<<<1, 32, 0, st>>>(dots, qq_dev + k, scal + 2, scal + 4); P2_COUNT_LAUNCH();
-        k_axpy4<<<nblk(n), kThreads, 0, st>>>((int)n, scal + 2, 1.0, gx, z); P2_COUNT_LAUNCH();
-        k = (k + 1) % m;
-        it++;
+        const unsigned blocks = nblk(n2, kBasisThreads);
+        if (f32) {
+            Corrections<float2> C{};
+            for (int j = 0; j < k; j++) { C.v[j] = (const float2 *)Z32[j].c[0]; C.y[j] = y[j]; }
+            k_basis_axpy<float2><<<blocks, kBasisThreads, 0, st>>>(n2, (double2 *)gx.c[0], C, k); P2_COUNT_LAUNCH();
+        } else {
+            Corrections<double2> C{};
+            for (int j = 0; j < k; j++) { C.v[j] = (const double2 *)Z64[j].c[0]; C.y[j] = y[j]; }
+            k_basis_axpy<double2><<<blocks, kBasisThreads, 0, st>>>(n2, (double2 *)gx.c[0], C, k); P2_COUNT_LAUNCH();
+        }
+        P2_CUDA_TRY(cudaGetLastError());
     }
     for (const auto &mk : vc_marks) {
         float t = 0;
@@ -1432,7 +1478,7 @@ p2_tune_info Solver::autotune(int trial_iters)
             prm.npost[0] = base_post / 2;
         }
     }
-    // GCR restart length: full solves of the chosen schedule with the
+    // GMRES restart length: full solves of the chosen schedule with the
     // configured length and with 12 (the directions stay allocated for the
     // longer one); the trials above stop before a restart shows its effect
     best.restart = restart;
@@ -1759,7 +1805,8 @@ double Solver::debug_time_stage(int stage, int l, int variant, int reps)
             } else if (stage == 1) {
                 rows0(gx, gr, f32 ? &L[0].r32 : nullptr, 0);
             } else if (stage == 4) {
-                rows0(Z[0], Q[0], nullptr, 1);
+                if (f32) rows0(Z32[0], W[1], nullptr, 1);
+                else rows0(Z64[0], W[1], nullptr, 1);
             } else if (stage == 2) {
                 Level &F = L[l], &Cl = L[l + 1];
                 if (f32)

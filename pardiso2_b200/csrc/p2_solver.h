@@ -224,12 +224,11 @@ class Solver {
     template <typename T>
     void capture_vcycle_graph();
     void set_nodes_device();
-    void dots_sync(const DotJobs &jobs);
     template <typename S>
     void rows0(const Vec4<S> &x, Vec4<double> &out, Vec4<float> *r32, int mode);
     void precondition();
     std::vector<cudaEvent_t> vc_ev;  // V-cycle timing events of a solve (reused)
-    double *qq_dev = nullptr;        // (Q_j, Q_j) of the stored directions
+    double residual_norm2();
     void debug_prepare();
     Grid3 grid3() const;
     void ensure_move_buffers(long nmark);
@@ -255,8 +254,14 @@ class Solver {
     LuGraph lu_graph;  // coarsest LU + inverse launch sequence
     int restart = 8;
     Vec4<double> gx, gb, gr;
-    std::vector<Vec4<double>> Z, Q;
-    double *partial = nullptr, *dots = nullptr, *scal = nullptr;
+    // GMRES basis W_0 .. W_m (FP64) with its squared norms ww, and the V-cycle's
+    // corrections Z_j in the cycle's own type
+    std::vector<Vec4<double>> W;
+    std::vector<Vec4<float>> Z32;
+    std::vector<Vec4<double>> Z64;
+    double *ww = nullptr, *hcol = nullptr;
+    double *partial = nullptr, *scal = nullptr;
+    unsigned *dticket = nullptr;  // last-block ticket of the outer loop's reductions (returns to zero)
     double *rpartial = nullptr;   // per-block partial sums of the fused restriction
     unsigned *rticket = nullptr;  // its last-block ticket (returns to zero)
     double *hdots_raw = nullptr;
