@@ -42,8 +42,18 @@ struct LuGraph {
     cudaGraphExec_t exec = nullptr;
     int n = 0, kl = -1, ku = -1;
     const double *A = nullptr, *Ainv = nullptr;
-    const int *ipiv = nullptr, *info = nullptr;
+    const int *ipiv = nullptr, *info = nullptr, *perm = nullptr;
     long long kernels = 0;
+};
+
+// Order of the coarsest free unknowns for the blocked inverse (p2_gj.cuh):
+// slot -> index in A's order (-1 padding) and back, and per panel the
+// velocity and pressure tiles it touches.
+constexpr int kGT = 64;  // tile edge and panel width
+struct GjPlan {
+    int nF = 0, n = 0, nv = 0;  // unknowns, padded size, padded velocity part
+    const int *perm = nullptr, *iperm = nullptr;
+    std::vector<int> tv, tq;
 };
 #define P2_COUNT_LAUNCH() (++p2::g_launches)
 

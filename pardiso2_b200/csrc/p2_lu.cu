@@ -1,5 +1,6 @@
-// Coarsest-level direct solve: FP64 LU with partial pivoting and its explicit
-// inverse, all on the device.
+// Coarsest-level direct solve: the explicit inverse in FP64, all on the device,
+// by blocked Gauss-Jordan elimination (p2_gj.cuh; gj_inverse below) or, where
+// that meets a zero pivot or fails its check, from an LU with partial pivoting.
 //
 // Replaces the MKL PARDISO call of the reference (pardiso/gaus3mg_SerieMG.c:
 // 64-309; phases 11/22/33 at 170/185/198).  The coarsest operator is reduced
@@ -25,9 +26,12 @@
 #include <cstdlib>
 #include <vector>
 
+#include "p2_gj.cuh"
 #include "p2_internal.cuh"
 
 namespace p2 {
+
+void d2f(cudaStream_t st, size_t n, const double *a, float *b);
 
 constexpr int kPB = 32;                                  // panel width
 constexpr int kMaxPanelBytes = 200 * 1024;               // shared-memory panel
@@ -43,6 +47,11 @@ constexpr int kMaxPanelRows = kMaxPanelBytes / (8 * kPB);  // 800 rows
 // rows are written back in that order: the result of a row-swapping panel
 // factorisation (partial pivoting, LAPACK getf2) of the same columns.
 constexpr int kTrackThreads = 1024;
+
+// Magnitude of a pivot candidate; a NaN counts as 0, so that every comparison
+// of the search is ordered and its winner is always a row of the panel.
+__device__ __forceinline__ double pivot_size(double v) { return v == v ? fabs(v) : 0.0; }
+
 static_assert(kMaxPanelRows <= kTrackThreads, "one thread per panel row");
 
 __global__ void __launch_bounds__(kTrackThreads) k_panel_track(double *A, int lda, int k0, int nb, int r1, int *ipiv,
@@ -62,7 +71,7 @@ __global__ void __launch_bounds__(kTrackThreads) k_panel_track(double *A, int ld
     const int row = threadIdx.x, lane = row & 31, w = row >> 5;
     bool live = row < m;  // not yet chosen as a pivot
     for (int jj = 0; jj < nb; jj++) {
-        double best = live ? fabs(P[(size_t)jj * m + row]) : -1.0;
+        double best = live ? pivot_size(P[(size_t)jj * m + row]) : -1.0;
         int bi = live ? row : 0x7fffffff;
         for (int o = 16; o > 0; o >>= 1) {
             double ov = __shfl_down_sync(0xffffffffu, best, o);
@@ -142,7 +151,7 @@ __global__ void __launch_bounds__(kRegPanelRows) k_panel_reg(double *A, int lda,
 #pragma unroll
     for (int jj = 0; jj < kPB; jj++) {
         const int buf = jj & 1;
-        double best = live ? fabs(v[jj]) : -1.0;
+        double best = live ? pivot_size(v[jj]) : -1.0;
         int bi = live ? row : 0x7fffffff;
         for (int o = 16; o > 0; o >>= 1) {
             double ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -525,13 +534,12 @@ struct LuTimer {
 
 // Factor the banded A (n x n, column-major, lower/upper half-bandwidths kl,
 // ku) in place and write its inverse into Ainv.  Returns 0 or the first
-// zero-pivot column + 1.  marks (optional, 2 events) are recorded after the
-// factorisation and after the forward half of the inverse.
+// zero-pivot column + 1.
 // panels per group in the backward half of the inverse
 constexpr int kInvGroup = 4;
 
 static void lu_issue(cudaStream_t st, double *A, int n, int kl, int ku, double *Ainv, int *d_ipiv, int *d_info,
-                     cudaEvent_t *marks, LuTimer &T)
+                     LuTimer &T)
 {
     const bool smem = kPB + kl <= kMaxPanelRows;
     P2_CUDA_TRY(cudaMemsetAsync(d_info, 0, sizeof(int), st));
@@ -564,7 +572,6 @@ static void lu_issue(cudaStream_t st, double *A, int n, int kl, int ku, double *
             T.end(2);
         }
     }
-    if (marks) P2_CUDA_TRY(cudaEventRecord(marks[0], st));
     // forward: replay (P_k, L_k) on the identity; rows [k0, r1) of the partial
     // product only have non-zeros in columns [0, r1)
     P2_CUDA_TRY(cudaMemsetAsync(Ainv, 0, sizeof(double) * (size_t)n * n, st));
@@ -581,7 +588,6 @@ static void lu_issue(cudaStream_t st, double *A, int n, int kl, int ku, double *
         if (r1 > cb) dgemm_sub(st, r1 - cb, r1, nb, A + (size_t)k0 * n + cb, n, Ainv + k0, n, Ainv + cb, n);
         T.end(2);
     }
-    if (marks) P2_CUDA_TRY(cudaEventRecord(marks[1], st));
     // backward: U X = Y with U's band (kl + ku above the diagonal), in groups
     // of kInvGroup panels: inside a group every panel's rows are solved and
     // propagated to the group's rows above it; then the rows above the group
@@ -611,7 +617,7 @@ static void lu_issue(cudaStream_t st, double *A, int n, int kl, int ku, double *
 }
 
 int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *Ainv, int *d_ipiv, int *d_info,
-                    cudaEvent_t *marks, LuGraph *cache, bool wait)
+                    LuGraph *cache)
 {
     kl = std::max(0, std::min(kl, n - 1));
     ku = std::max(0, std::min(ku, n - 1));
@@ -628,7 +634,7 @@ int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *A
             P2_CUDA_TRY(cudaEventCreate(&T.b));
         }
     }
-    if (cache && !T.on && !marks) {
+    if (cache && !T.on) {
         // the ~800 dependent launches replayed as one graph; captured again
         // only when the size, the band or the buffers change
         const bool hit = cache->exec && cache->n == n && cache->kl == kl && cache->ku == ku && cache->A == A &&
@@ -639,7 +645,7 @@ int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *A
             cudaGraph_t graph;
             long long before = g_launches;
             P2_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            lu_issue(st, A, n, kl, ku, Ainv, d_ipiv, d_info, nullptr, T);
+            lu_issue(st, A, n, kl, ku, Ainv, d_ipiv, d_info, T);
             P2_CUDA_TRY(cudaStreamEndCapture(st, &graph));
             cache->kernels = g_launches - before;
             g_launches = before;
@@ -652,7 +658,7 @@ int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *A
         P2_CUDA_TRY(cudaGraphLaunch(cache->exec, st));
         g_launches += cache->kernels;
     } else {
-        lu_issue(st, A, n, kl, ku, Ainv, d_ipiv, d_info, marks, T);
+        lu_issue(st, A, n, kl, ku, Ainv, d_ipiv, d_info, T);
     }
     if (T.on) {
         std::fprintf(stderr, "p2cuda LU timing: panel %.3f ms (%d), lower TRSM %.3f ms (%d), GEMM %.3f ms (%d), "
@@ -662,10 +668,78 @@ int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *A
         cudaEventDestroy(T.b);
     }
     int info = 0;
-    if (!wait) return 0;  // the caller reads d_info once the stream has finished
     P2_CUDA_TRY(cudaMemcpyAsync(&info, d_info, sizeof(int), cudaMemcpyDeviceToHost, st));
     P2_CUDA_TRY(cudaStreamSynchronize(st));
     return info;
+}
+
+// Inverse of A (nF x nF, column-major) into X (n x n in the plan's order, see
+// p2_gj.cuh) and its float copy Xf (or null); d_flag is set when a pivot is not
+// positive or the check of the inverse fails.  A is only read.
+static void gj_issue(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag)
+{
+    const int n = P.n, nt = n / kGT;
+    double *Lb = work, *Ub = Lb + (size_t)kGT * n, *D = Ub + (size_t)kGT * n, *y = D + 4 * kGT * kGT;
+    P2_CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), st));
+    k_gj_gather<<<dim3((n + 255) / 256, n), 256, 0, st>>>(n, P.nF, P.perm, A, X); P2_COUNT_LAUNCH();
+    k_gj_first<<<1, kGThreads, 0, st>>>(X, n, D, d_flag); P2_COUNT_LAUNCH();
+    for (int p = 0; p < nt; p++) {
+        const GjTiles T{P.tv[p], P.tq[p], P.nv / kGT};
+        double *Dp = D + (p & 1) * 2 * kGT * kGT, *Dn = D + ((p + 1) & 1) * 2 * kGT * kGT;
+        const int next = p + 1 < nt ? p + 1 : -1;
+        k_gj_panel<<<2 * T.count(), kGThreads, kGjSmem, st>>>(X, n, p, T, Dp, Lb, Ub); P2_COUNT_LAUNCH();
+        k_gj_update<<<dim3(T.count(), T.count()), kGThreads, kGjSmem, st>>>(X, n, p, next, T, Lb, Ub, Dn, d_flag); P2_COUNT_LAUNCH();
+    }
+    k_gj_check_x<<<(n + 31) / 32, 32 * kCheckWarps, 0, st>>>(n, P.perm, X, y); P2_COUNT_LAUNCH();
+    k_gj_check_a<<<(P.nF + 31) / 32, 32 * kCheckWarps, 0, st>>>(P.nF, P.iperm, A, y, d_flag); P2_COUNT_LAUNCH();
+    if (Xf) d2f(st, (size_t)n * n, X, Xf);
+    P2_CUDA_TRY(cudaGetLastError());
+}
+
+size_t gj_work_doubles(int n) { return (size_t)2 * kGT * n + 4 * kGT * kGT + n; }
+
+// gj_issue replayed as one graph, captured again only when the plan or the
+// buffers change.
+void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
+                LuGraph *cache)
+{
+    // per-device attributes, set on the current device (host-side calls)
+    P2_CUDA_TRY(cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
+    P2_CUDA_TRY(cudaFuncSetAttribute(k_gj_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
+    const bool hit = cache->exec && cache->n == P.n && cache->A == A && cache->Ainv == X && cache->info == d_flag &&
+                     cache->perm == P.perm;
+    if (!hit) {
+        if (cache->exec) cudaGraphExecDestroy(cache->exec);
+        cache->exec = nullptr;
+        cudaGraph_t graph;
+        const long long before = g_launches;
+        P2_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        gj_issue(st, A, P, X, Xf, work, d_flag);
+        P2_CUDA_TRY(cudaStreamEndCapture(st, &graph));
+        cache->kernels = g_launches - before;
+        g_launches = before;
+        const cudaError_t e = cudaGraphInstantiate(&cache->exec, graph, 0);
+        cudaGraphDestroy(graph);
+        P2_CUDA_TRY(e);
+        cache->n = P.n; cache->A = A; cache->Ainv = X; cache->info = d_flag; cache->perm = P.perm;
+    }
+    P2_CUDA_TRY(cudaGraphLaunch(cache->exec, st));
+    g_launches += cache->kernels;
+}
+
+// X (n x n in the plan's order, identity on the padding) from the inverse B
+// in A's order
+__global__ void k_permute_inverse(int n, int nF, const int *perm, const double *B, double *X)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    if (r >= n) return;
+    const int pr = perm[r], pc = perm[c];
+    X[(size_t)c * n + r] = pr >= 0 && pc >= 0 ? B[(size_t)pc * nF + pr] : (r == c ? 1.0 : 0.0);
+}
+void permute_inverse(cudaStream_t st, const GjPlan &P, const double *B, double *X)
+{
+    k_permute_inverse<<<dim3((P.n + 255) / 256, P.n), 256, 0, st>>>(P.n, P.nF, P.perm, B, X); P2_COUNT_LAUNCH();
+    P2_CUDA_TRY(cudaGetLastError());
 }
 
 void d2f(cudaStream_t st, size_t n, const double *a, float *b)

@@ -32,38 +32,42 @@ namespace p2 {
 
 constexpr int kProbes = 4 * 125;  // coarsest-operator probes: 125 colour classes x 4 components
 int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *Ainv, int *d_ipiv, int *d_info,
-                    cudaEvent_t *marks, LuGraph *cache, bool wait = true);
+                    LuGraph *cache);
 // sweeps of the diagonal cell smoother on the coarsest level standing in for
 // its direct solve while the LU is still running
 constexpr int kCoarseApxSweeps = 16;
 // cell planes per block of the fused sweep (each block starts 3 planes early)
 constexpr int kSweepChunk = 32;
 // Outer iterations that use the smoothed coarsest level: kOverlapScale *
-// nF / n0, the LU's latency-bound panel chain (about linear in nF) over the
-// fine work of one iteration (linear in n0), fixed from the grid sizes so
-// that the iterates do not depend on timing (10 at 65^3, 2 at 129^3, 0 at
-// 257^3 with nF = 6912); none on grids of fewer than four levels, where the
+// nF / n0, the inverse's time over the fine work of one iteration (linear in
+// n0), fixed from the grid sizes so that the iterates do not depend on timing
+// (5 at 65^3, where the inverse takes 4.3 ms, 1 at 129^3, 0 at 257^3, all with
+// nF = 3644); none on grids of fewer than four levels, where the
 // coarsest level is too large a part of the problem for smoothing to stand
 // in for it.  The solve waits for the LU at that iteration if it is still
 // running.
 constexpr double kOverlapScale = 400.0;
 constexpr int kOverlapMax = 16;
 void d2f(cudaStream_t st, size_t n, const double *a, float *b);
+size_t gj_work_doubles(int n);
+void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
+                LuGraph *cache);
+void permute_inverse(cudaStream_t st, const GjPlan &P, const double *B, double *X);
 
 static inline unsigned nblk(long n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
 
 // Launch with programmatic stream serialization (see pdl_enter): kernels
 // launched this way start with pdl_enter().
 template <typename... KArgs, typename... Args>
-static void pdl_launch(cudaStream_t st, dim3 grid, dim3 block, void (*kern)(KArgs...), Args &&...args)
+static void pdl_launch_smem(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kern)(KArgs...), Args &&...args)
 {
 #ifdef P2_NO_PDL
-    kern<<<grid, block, 0, st>>>(std::forward<Args>(args)...);
+    kern<<<grid, block, smem, st>>>(std::forward<Args>(args)...);
 #else
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -73,6 +77,11 @@ static void pdl_launch(cudaStream_t st, dim3 grid, dim3 block, void (*kern)(KArg
     P2_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
 #endif
     P2_COUNT_LAUNCH();
+}
+template <typename... KArgs, typename... Args>
+static void pdl_launch(cudaStream_t st, dim3 grid, dim3 block, void (*kern)(KArgs...), Args &&...args)
+{
+    pdl_launch_smem(st, grid, block, 0, kern, std::forward<Args>(args)...);
 }
 
 void *DeviceArena::alloc(size_t bytes)
@@ -231,6 +240,7 @@ Solver::~Solver()
     if (st_lu) cudaStreamSynchronize(st_lu);
     drop_graphs();
     if (lu_graph.exec) cudaGraphExecDestroy(lu_graph.exec);
+    if (lu_graph_pivoted.exec) cudaGraphExecDestroy(lu_graph_pivoted.exec);
     arena.release();
     grid_arena.release();
     marker_arena.release();
@@ -669,8 +679,46 @@ void Solver::build_coarse_index()
     }
     nF = (int)fre.size();
     coarse_col = col;
-    d_free = upload(arena, fre);
     d_colmap = upload(arena, col);
+    // slots of the inverse: velocities, then pressures, each by z-plane (the
+    // natural order) and padded to whole tiles
+    {
+        const int plane_nodes = C.nx * C.ny;
+        std::vector<int> part[2], perm, iperm(nF, -1), list, slot_of(C.n * 4, -1);
+        for (int q = 0; q < nF; q++) part[(fre[q] & 3) == 0].push_back(q);
+        for (int h = 0; h < 2; h++) {
+            for (int q : part[h]) perm.push_back(q);
+            while (perm.size() % kGT) perm.push_back(-1);
+            if (h == 0) gj.nv = (int)perm.size();
+        }
+        gj.nF = nF;
+        gj.n = (int)perm.size();
+        for (int r = 0; r < gj.n; r++) {
+            list.push_back(perm[r] >= 0 ? fre[perm[r]] : -1);
+            if (perm[r] < 0) continue;
+            iperm[perm[r]] = r;
+            slot_of[fre[perm[r]]] = r;
+        }
+        // tiles within two planes of the ones eliminated so far
+        const int nt = gj.n / kGT, nvt = gj.nv / kGT;
+        gj.tv.assign(nt, nvt);
+        gj.tq.assign(nt, nt - nvt);
+        auto reach = [&](const std::vector<int> &v, int plane) {
+            size_t c = v.size();
+            while (c > 0 && (fre[v[c - 1]] >> 2) / plane_nodes > plane) c--;
+            return (int)((c + kGT - 1) / kGT);
+        };
+        for (int p = 0; p < nvt; p++) {
+            const size_t last = std::min<size_t>((size_t)(p + 1) * kGT, part[0].size()) - 1;
+            const int plane = (fre[part[0][last]] >> 2) / plane_nodes + 2;
+            gj.tv[p] = std::max(reach(part[0], plane), std::min(p + 2, nvt));
+            gj.tq[p] = p + 1 == nvt ? nt - nvt : reach(part[1], plane);
+        }
+        gj.perm = upload(arena, perm);
+        gj.iperm = upload(arena, iperm);
+        d_slots = upload(arena, list);
+        d_slot_of = upload(arena, slot_of);
+    }
     // resolved boundary rows of the coarsest level as a dense per-unknown map
     std::vector<int> rt(C.n * 4, -2);
     std::vector<float> rk(C.n * 4, 0.0f);
@@ -681,8 +729,10 @@ void Solver::build_coarse_index()
     d_crt = upload(arena, rt);
     d_crk = upload(arena, rk);
     A_c = (double *)arena.alloc(sizeof(double) * (size_t)nF * nF);
-    Ainv64 = (double *)arena.alloc(sizeof(double) * (size_t)nF * nF);
-    Ainv32 = (float *)arena.alloc(sizeof(float) * (size_t)nF * nF);
+    Ainv64 = (double *)arena.alloc(sizeof(double) * (size_t)gj.n * gj.n);
+    Ainv32 = (float *)arena.alloc(sizeof(float) * (size_t)gj.n * gj.n);
+    gj_work = (double *)arena.alloc(sizeof(double) * gj_work_doubles(gj.n));
+    Ainv_natural = nullptr;
     d_ipiv = (int *)arena.alloc(sizeof(int) * nF);
     d_info = (int *)arena.alloc(sizeof(int) * 4);
     probes = (double *)arena.alloc(sizeof(double) * (size_t)C.n * 4 * kProbes);
@@ -693,10 +743,8 @@ void Solver::build_coarse_index()
         h_bw_keep.reset(p, [](int *q) { cudaFreeHost(q); });
         h_bw = p;
     }
-    cb64 = (double *)arena.alloc(sizeof(double) * nF);
-    cx64 = (double *)arena.alloc(sizeof(double) * nF);
-    cb32 = (float *)arena.alloc(sizeof(float) * nF);
-    cx32 = (float *)arena.alloc(sizeof(float) * nF);
+    cpart64 = (double *)arena.alloc(sizeof(double) * gj.n * gemv_splits<double>(gj.n));
+    cpart32 = (float *)arena.alloc(sizeof(float) * gj.n * gemv_splits<float>(gj.n));
 }
 
 // ---------------------------------------------------------------------------
@@ -782,47 +830,47 @@ void Solver::coarse_setup()
     k_probe_build<<<grid, kThreads, 0, st>>>(C.nx, C.ny, C.nz, d_colmap, d_crt, d_crk, probes); P2_COUNT_LAUNCH();
     k_probe_rows<<<grid, kThreads, 0, st>>>(Lc, probes, d_colmap, A_c, nF, d_bw); P2_COUNT_LAUNCH();
     P2_CUDA_TRY(cudaGetLastError());
-    P2_CUDA_TRY(cudaMemcpyAsync(h_bw, d_bw, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
-    P2_CUDA_TRY(cudaStreamSynchronize(st));
-    if (!verbose) {
-        // The LU and the inverse run on their own stream (st has no work in
-        // flight after the synchronisation above); the solve goes on with a
-        // smoothed coarsest level for lu_overlap_iters outer iterations.
-        band_lu_inverse(st_lu, A_c, nF, h_bw[0], h_bw[1], Ainv64, d_ipiv, d_info, nullptr, &lu_graph, false);
-        d2f(st_lu, (size_t)nF * nF, Ainv64, Ainv32);
-        P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
-        lu_pending = true;
-        lu_overlap_iters = L.size() < 4 ? 0
-                           : (int)std::min<double>(kOverlapMax, std::floor(kOverlapScale * nF / (double)L[0].n + 0.5));
-        return;
-    }
-    P2_CUDA_TRY(cudaEventRecord(ev[5], st));
-    int info = band_lu_inverse(st, A_c, nF, h_bw[0], h_bw[1], Ainv64, d_ipiv, d_info, verbose ? ev + 6 : nullptr,
-                               &lu_graph);
-    if (verbose) {
-        float t0 = 0, t1 = 0, t2 = 0;
-        P2_CUDA_TRY(cudaEventElapsedTime(&t0, ev[0], ev[5]));
-        P2_CUDA_TRY(cudaEventElapsedTime(&t1, ev[5], ev[6]));
-        P2_CUDA_TRY(cudaEventElapsedTime(&t2, ev[6], ev[7]));
-        std::fprintf(stderr, "p2cuda: coarsest nF %d band kl %d ku %d; node fields + probing %.3f ms, "
-                     "factorisation %.3f ms, inverse (forward) %.3f ms\n", nF, h_bw[0], h_bw[1], t0, t1, t2);
-    }
-    if (info) throw Error(P2_ERR_SINGULAR, "zero pivot in the coarsest LU at column " + std::to_string(info));
-    d2f(st, (size_t)nF * nF, Ainv64, Ainv32);
+    // The inverse runs on its own stream; the solve goes on with a smoothed
+    // coarsest level for lu_overlap_iters outer iterations.
+    P2_CUDA_TRY(cudaEventRecord(ev_lu, st));
+    P2_CUDA_TRY(cudaStreamWaitEvent(st_lu, ev_lu, 0));
+    gj_inverse(st_lu, A_c, gj, Ainv64, prm.precision == 0 ? Ainv32 : nullptr, gj_work, d_info, &lu_graph);
+    P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
+    lu_pending = true;
+    lu_overlap_iters = L.size() < 4 ? 0
+                       : (int)std::min<double>(kOverlapMax, std::floor(kOverlapScale * nF / (double)L[0].n + 0.5));
 }
 
-// The overlapped LU: wait for it, check its pivots and order the solve's
-// stream after it.
+// The inverse by the pivoted band LU (A_c is overwritten), brought into the
+// slots' order; its buffer is allocated on first use.
+void Solver::lu_pivoted()
+{
+    P2_CUDA_TRY(cudaMemcpyAsync(h_bw, d_bw, sizeof(int) * 2, cudaMemcpyDeviceToHost, st_lu));
+    P2_CUDA_TRY(cudaStreamSynchronize(st_lu));
+    if (!Ainv_natural) Ainv_natural = (double *)arena.alloc(sizeof(double) * (size_t)nF * nF);
+    const int info = band_lu_inverse(st_lu, A_c, nF, h_bw[0], h_bw[1], Ainv_natural, d_ipiv, d_info, &lu_graph_pivoted);
+    if (info) throw Error(P2_ERR_SINGULAR, "zero pivot in the coarsest LU at column " + std::to_string(info));
+    permute_inverse(st_lu, gj, Ainv_natural, Ainv64);
+    d2f(st_lu, (size_t)gj.n * gj.n, Ainv64, Ainv32);
+    P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
+    P2_CUDA_TRY(cudaStreamWaitEvent(st, ev_lu, 0));
+    lu_pending = false;
+}
+
+// The overlapped inverse: wait for it, order the solve's stream after it and
+// look at its flag; an inverse that failed its check is done again with
+// pivoting.
 void Solver::lu_finish()
 {
     if (!lu_pending) return;
     P2_CUDA_TRY(cudaEventSynchronize(ev_lu));
-    int info = 0;
-    P2_CUDA_TRY(cudaMemcpyAsync(&info, d_info, sizeof(int), cudaMemcpyDeviceToHost, st_lu));
+    int flag = 0;
+    P2_CUDA_TRY(cudaMemcpyAsync(&flag, d_info, sizeof(int), cudaMemcpyDeviceToHost, st_lu));
     P2_CUDA_TRY(cudaStreamSynchronize(st_lu));
     P2_CUDA_TRY(cudaStreamWaitEvent(st, ev_lu, 0));
     lu_pending = false;
-    if (info) throw Error(P2_ERR_SINGULAR, "zero pivot in the coarsest LU at column " + std::to_string(info));
+    if (verbose) std::fprintf(stderr, "p2cuda: coarsest inverse n %d (padded %d) flag %d\n", nF, gj.n, flag);
+    if (flag) lu_pivoted();
 }
 
 // Stand-in for the coarsest direct solve: x = 0, then sweeps of the diagonal
@@ -847,13 +895,14 @@ void Solver::coarse_solve(Vec4<T> &b, Vec4<T> &x)
         return;
     }
     Level &C = L.back();
-    T *bF = std::is_same<T, double>::value ? (T *)cb64 : (T *)cb32;
-    T *xF = std::is_same<T, double>::value ? (T *)cx64 : (T *)cx32;
     const T *Ai = std::is_same<T, double>::value ? (const T *)Ainv64 : (const T *)Ainv32;
-    for (int c = 0; c < 4; c++) P2_CUDA_TRY(cudaMemsetAsync(x.c[c], 0, sizeof(T) * C.n, st));
-    pdl_launch(st, nblk(nF), kThreads, k_coarse_gather<T>, nF, (const int *)d_free, b, bF);
-    pdl_launch(st, (nF + 31) / 32, 256, k_gemv<T>, nF, Ai, (const T *)bF, xF);
-    pdl_launch(st, nblk(nF), kThreads, k_coarse_scatter<T>, nF, (const int *)d_free, (const T *)xF, x);
+    T *part = std::is_same<T, double>::value ? (T *)cpart64 : (T *)cpart32;
+    const int splits = gemv_splits<T>(gj.n), chunk = (gj.n + splits - 1) / splits;
+    const dim3 grid((gj.n + gemv_rows<T>() - 1) / gemv_rows<T>(), splits);
+    pdl_launch_smem(st, grid, dim3(32 * kGemvWarps), sizeof(T) * chunk, k_gemv_split<T>, gj.n, Ai, (const int *)d_slots, b,
+                    part, chunk);
+    pdl_launch(st, nblk(4L * C.n), kThreads, k_coarse_write<T>, C.n, gj.n, splits, (const int *)d_slot_of,
+               (const T *)part, x);
     bc_set<T>((int)L.size() - 1, x, b);
 }
 
@@ -1241,13 +1290,6 @@ p2_solve_info Solver::solve()
     factor_cells();
     coarse_setup();
     P2_CUDA_TRY(cudaEventRecord(ev[1], st));
-    if (verbose) {
-        float tb = 0;
-        P2_CUDA_TRY(cudaEventSynchronize(ev[1]));
-        P2_CUDA_TRY(cudaEventElapsedTime(&tb, ev[7], ev[1]));
-        std::fprintf(stderr, "p2cuda: inverse (backward) + FP32 copy %.3f ms; V-cycle graph %lld kernels\n", tb,
-                     graphs[prm.precision == 0 ? 0 : 1].kernels);
-    }
     // b-norm of the pinned system: every row but the pin cell's, plus the pin value
     const bool f32 = prm.precision == 0;
     const long n2 = 2L * n;

@@ -269,7 +269,12 @@ class Solver {
     // coarsest level
     int nF = 0;
     std::vector<int> coarse_col;
-    int *d_free = nullptr, *d_colmap = nullptr, *d_crt = nullptr;
+    int *d_colmap = nullptr, *d_crt = nullptr;
+    GjPlan gj;
+    int *d_slots = nullptr, *d_slot_of = nullptr;  // unknown of each slot of the inverse (-1 padding), and back
+    double *gj_work = nullptr, *Ainv_natural = nullptr;
+    LuGraph lu_graph_pivoted;
+    void lu_pivoted();
     float *d_crk = nullptr;
     double *A_c = nullptr, *Ainv64 = nullptr;
     float *Ainv32 = nullptr;
@@ -277,8 +282,8 @@ class Solver {
     double *probes = nullptr;
     int *d_bw = nullptr, *h_bw = nullptr;  // band of the coarsest operator (kl, ku)
     std::shared_ptr<int> h_bw_keep;
-    double *cb64 = nullptr, *cx64 = nullptr;
-    float *cb32 = nullptr, *cx32 = nullptr;
+    double *cpart64 = nullptr;             // partial products of the coarsest solve
+    float *cpart32 = nullptr;
 };
 
 }  // namespace p2
