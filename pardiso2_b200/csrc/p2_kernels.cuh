@@ -116,73 +116,6 @@ __global__ void k_bc_set_chain(int nbc, const int *bu, const int *bt, const floa
 }
 
 // ---------------------------------------------------------------------------
-// One colour pass of the cell-block smoother (diagonal Vanka / SCGS) over the
-// cells with (i+j+k)&1 == col.  Each cell corrects its six face velocities and
-// its pressure together with the velocity block replaced by its diagonal:
-//   d_v dv_v + g_v dp = r_v,  sum_v c_v dv_v = r_p.
-// Every cell of the colour reads the state from before the pass: velocities
-// are read from vin and written to vout (each face belongs to exactly one
-// cell of each colour), the pressure is updated in place (a cell's pressure is
-// read only by its own face rows among the cells of one colour).
-template <typename T>
-__device__ __forceinline__ void vanka_item(const LevelView<T> &L, T *P, const Vec4<T> &vin, const Vec4<T> &vout,
-                                           const Vec4<T> &b, T omega, int col, long t)
-{
-    int half = (L.ny) / 2;  // >= number of cells of one colour on a y-line
-    long lines = (long)(L.nx - 1) * (L.nz - 1);
-    if (t >= lines * half) return;
-    int jj = (int)(t % half);
-    long line = t / half;
-    int i = 1 + (int)(line % (L.nx - 1)), k = 1 + (int)(line / (L.nx - 1));
-    int j0 = (((1 + i + k) & 1) == col) ? 1 : 2;
-    int j = j0 + 2 * jj;
-    if (j > L.ny - 1) return;
-    Fields<T, T> x{P, vin.c[1], vin.c[2], vin.c[3]};
-    int u = P2IDX(L, i, j, k);
-    bool pbc = (L.bcm[u] & BC_P) != 0;
-    int fi[6], fc[6];
-    T g[6], cc[6], r[6], d[6];
-    fc[0] = 1; fi[0] = P2IDX(L, i - 1, j - 1, k - 1); g[0] = -L.ax.ihc[i - 1]; cc[0] = -L.ax.ih[i];
-    fc[1] = 1; fi[1] = P2IDX(L, i, j - 1, k - 1);     g[1] = L.ax.ihc[i];      cc[1] = L.ax.ih[i];
-    fc[2] = 2; fi[2] = P2IDX(L, i - 1, j - 1, k - 1); g[2] = -L.ay.ihc[j - 1]; cc[2] = -L.ay.ih[j];
-    fc[3] = 2; fi[3] = P2IDX(L, i - 1, j, k - 1);     g[3] = L.ay.ihc[j];      cc[3] = L.ay.ih[j];
-    fc[4] = 3; fi[4] = P2IDX(L, i - 1, j - 1, k - 1); g[4] = -L.az.ihc[k - 1]; cc[4] = -L.az.ih[k];
-    fc[5] = 3; fi[5] = P2IDX(L, i - 1, j - 1, k);     g[5] = L.az.ihc[k];      cc[5] = L.az.ih[k];
-    const int ofs[6][3] = {{-1, -1, -1}, {0, -1, -1}, {-1, -1, -1}, {-1, 0, -1}, {-1, -1, -1}, {-1, -1, 0}};
-    T num = 0, den = 0;
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        int a = i + ofs[q][0], bb = j + ofs[q][1], c = k + ofs[q][2];
-        d[q] = 0;
-        r[q] = 0;
-        if (L.bcm[fi[q]] & (1 << fc[q])) continue;
-        T ax;
-        if (fc[q] == 1) ax = row_vx(L, x, a, bb, c, &d[q]);
-        else if (fc[q] == 2) ax = row_vy(L, x, a, bb, c, &d[q]);
-        else ax = row_vz(L, x, a, bb, c, &d[q]);
-        r[q] = b.c[fc[q]][fi[q]] - ax;
-        num += cc[q] * r[q] / d[q];
-        den += cc[q] * g[q] / d[q];
-    }
-    T dp = 0;
-    if (!pbc && den != (T)0) {
-        T rp = b.c[0][u] - row_p(L, x, i, j, k);
-        dp = (num - rp) / den;
-        P[u] += omega * dp;
-    }
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        if (d[q] != (T)0) vout.c[fc[q]][fi[q]] = vin.c[fc[q]][fi[q]] + omega * (r[q] - g[q] * dp) / d[q];
-    }
-}
-template <typename T>
-__global__ void k_vanka(LevelView<T> L, T *P, Vec4<T> vin, Vec4<T> vout, Vec4<T> b, T omega, int col)
-{
-    pdl_enter();
-    vanka_item(L, P, vin, vout, b, omega, col, (long)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// ---------------------------------------------------------------------------
 // Full cell-block variant: the cell's 6 face velocities and its pressure are
 // solved together with the exact 7x7 cell system
 //   [M g; cc^T 0] [dv; dp] = [r; rp],
@@ -346,6 +279,50 @@ __global__ void __launch_bounds__(128) k_vanka_full(LevelView<T> L, T *P, Vec4<T
         if (act[q]) vout.c[fc[q]][fi[q]] = vin.c[fc[q]][fi[q]] + omega * (y1[q] - dp * y2[q]);
 }
 
+// Viscosities a cell's rows use, in the order of cell_eta_offset: the cell
+// itself, its six neighbours (low, high x; y; z), its four edges of each
+// orientation.
+constexpr int kCellEta = 19;
+
+// Field (0 ec, 1 exy, 2 exz, 3 eyz) and node offset from the cell's low corner
+// F = (i-1, j-1, k-1) of viscosity q (y stride 1, x stride sy, z stride sz).
+__device__ __forceinline__ int cell_eta_offset(int q, int sy, int sz, int &field)
+{
+    field = q < 7 ? 0 : (q - 7) / 4 + 1;
+    const int u = sz + sy + 1, e = (q - 7) & 3;
+    switch (q) {
+    case 0: return u;
+    case 1: return u - sy;
+    case 2: return u + sy;
+    case 3: return u - 1;
+    case 4: return u + 1;
+    case 5: return u - sz;
+    case 6: return u + sz;
+    default: break;
+    }
+    // edge (lo, hi) along the two axes across it: xy 00 01 (y) 10 (x) 11, xz 00 01 (z) 10 (x) 11, yz 00 01 (z) 10 (y) 11
+    const int first = field == 3 ? 1 : sy, second = field == 1 ? 1 : sz;
+    return (e & 2 ? first : 0) + (e & 1 ? second : 0);
+}
+
+// Viscosities of a cell from the level's fields.
+template <typename T>
+struct LevelEta {
+    const LevelView<T> &L;
+    int F;
+    __device__ __forceinline__ T operator()(int q) const
+    {
+        int f;
+        const int o = F + cell_eta_offset(q, L.ny, L.nx * L.ny, f);
+        return eta_at(L, f == 0 ? L.ec : (f == 1 ? L.exy : (f == 2 ? L.exz : L.eyz)), o);
+    }
+};
+// Unknowns that no thread of the launch writes.
+struct LoadConst {
+    template <typename T>
+    __device__ __forceinline__ T operator()(const T *p) const { return __ldg(p); }
+};
+
 // Momentum parts (A v + grad p) of the six face rows of cell (i, j, k) from
 // shared stresses, and the cell's divergence: the cell's three normal
 // stresses from one set of strain rates, the six neighbour cells' normal
@@ -353,88 +330,126 @@ __global__ void __launch_bounds__(128) k_vanka_full(LevelView<T> L, T *P, Vec4<T
 // each.  Every velocity, viscosity and pressure is loaded once, addressed
 // from the cell's low corner F = (i-1, j-1, k-1) (y stride 1, x stride ny, z
 // stride nx*ny); the deviatoric third is a multiplication by 1/3.  The same
-// terms as row_vx/row_vy/row_vz up to rounding.
-template <typename T>
-__device__ __forceinline__ void cell_rows(const LevelView<T> &L, const Fields<T, T> &x, int i, int j, int k,
-                                          const int fi[6], T ax[6], T &div)
+// terms as row_vx/row_vy/row_vz up to rounding.  kDiag: also the rows'
+// diagonals (diag_vx .. diag_vz) in d.
+template <typename T, bool kDiag, typename Eta, typename Load>
+__device__ __forceinline__ void cell_rows(const Axis<T> &AX, const Axis<T> &AY, const Axis<T> &AZ, int sy, int sz,
+                                          const Fields<T, T> &x, int i, int j, int k, int F, const Eta &eta,
+                                          const Load &load, T ax[6], T &div, T *d)
 {
-    const int sy = L.ny, sz = L.nx * L.ny;
-    const int F = fi[0];
     const T *vx = x.vx + F, *vy = x.vy + F, *vz = x.vz + F;
     // velocities around the cell (offsets from F)
-    const T vx0 = __ldg(vx), vxX = __ldg(vx + sy), vxXX = __ldg(vx + 2 * sy), vxm = __ldg(vx - sy);
-    const T vxY = __ldg(vx + 1), vxy_ = __ldg(vx - 1), vxXY = __ldg(vx + sy + 1), vxXy = __ldg(vx + sy - 1);
-    const T vxZ = __ldg(vx + sz), vxz_ = __ldg(vx - sz), vxXZ = __ldg(vx + sy + sz), vxXz = __ldg(vx + sy - sz);
-    const T vy0 = __ldg(vy), vyY = __ldg(vy + 1), vyYY = __ldg(vy + 2), vym = __ldg(vy - 1);
-    const T vyX = __ldg(vy + sy), vyx_ = __ldg(vy - sy), vyXY = __ldg(vy + sy + 1), vyxY = __ldg(vy - sy + 1);
-    const T vyZ = __ldg(vy + sz), vyz_ = __ldg(vy - sz), vyYZ = __ldg(vy + 1 + sz), vyYz = __ldg(vy + 1 - sz);
-    const T vz0 = __ldg(vz), vzZ = __ldg(vz + sz), vzZZ = __ldg(vz + 2 * sz), vzm = __ldg(vz - sz);
-    const T vzX = __ldg(vz + sy), vzx_ = __ldg(vz - sy), vzXZ = __ldg(vz + sy + sz), vzxZ = __ldg(vz - sy + sz);
-    const T vzY = __ldg(vz + 1), vzy_ = __ldg(vz - 1), vzYZ = __ldg(vz + 1 + sz), vzyZ = __ldg(vz - 1 + sz);
+    const T vx0 = load(vx), vxX = load(vx + sy), vxXX = load(vx + 2 * sy), vxm = load(vx - sy);
+    const T vxY = load(vx + 1), vxy_ = load(vx - 1), vxXY = load(vx + sy + 1), vxXy = load(vx + sy - 1);
+    const T vxZ = load(vx + sz), vxz_ = load(vx - sz), vxXZ = load(vx + sy + sz), vxXz = load(vx + sy - sz);
+    const T vy0 = load(vy), vyY = load(vy + 1), vyYY = load(vy + 2), vym = load(vy - 1);
+    const T vyX = load(vy + sy), vyx_ = load(vy - sy), vyXY = load(vy + sy + 1), vyxY = load(vy - sy + 1);
+    const T vyZ = load(vy + sz), vyz_ = load(vy - sz), vyYZ = load(vy + 1 + sz), vyYz = load(vy + 1 - sz);
+    const T vz0 = load(vz), vzZ = load(vz + sz), vzZZ = load(vz + 2 * sz), vzm = load(vz - sz);
+    const T vzX = load(vz + sy), vzx_ = load(vz - sy), vzXZ = load(vz + sy + sz), vzxZ = load(vz - sy + sz);
+    const T vzY = load(vz + 1), vzy_ = load(vz - 1), vzYZ = load(vz + 1 + sz), vzyZ = load(vz - 1 + sz);
     const T third = (T)(1.0 / 3.0), two = (T)2.0;
-    const T hx0 = L.ax.ih[i - 1], hx1 = L.ax.ih[i], hx2 = L.ax.ih[i + 1];
-    const T hy0 = L.ay.ih[j - 1], hy1 = L.ay.ih[j], hy2 = L.ay.ih[j + 1];
-    const T hz0 = L.az.ih[k - 1], hz1 = L.az.ih[k], hz2 = L.az.ih[k + 1];
-    const int u = F + sz + sy + 1;
+    const T hx0 = AX.ih[i - 1], hx1 = AX.ih[i], hx2 = AX.ih[i + 1];
+    const T hy0 = AY.ih[j - 1], hy1 = AY.ih[j], hy2 = AY.ih[j + 1];
+    const T hz0 = AZ.ih[k - 1], hz1 = AZ.ih[k], hz2 = AZ.ih[k + 1];
+    // In FP32 the viscosities and pressures are loaded here too, so that all of a
+    // cell's loads are in flight together; in FP64 that costs too many registers.
+    constexpr bool kAhead = sizeof(T) == 4;
+    const T *pp = x.p + F + sz + sy + 1;
+    T en[kAhead ? kCellEta : 1], pn[kAhead ? 7 : 1];
+    const int po[7] = {0, -sy, sy, -1, 1, -sz, sz};
+    if constexpr (kAhead) {
+#pragma unroll
+        for (int q = 0; q < 7; q++) pn[q] = load(pp + po[q]);
+#pragma unroll
+        for (int q = 0; q < kCellEta; q++) en[q] = eta(q);
+    }
+    auto E = [&](int q) {
+        if constexpr (kAhead) return en[q];
+        else return eta(q);
+    };
+    auto PR = [&](int q) {
+        if constexpr (kAhead) return pn[q];
+        else return load(pp + po[q]);
+    };
     // own cell
     const T exx = (vxX - vx0) * hx1, eyy = (vyY - vy0) * hy1, ezz = (vzZ - vz0) * hz1;
     div = exx + eyy + ezz;
-    const T E2 = two * eta_at(L, L.ec, u);
+    const T E2 = two * E(0);
     const T s0 = E2 * (exx - div * third), s1 = E2 * (eyy - div * third), s2 = E2 * (ezz - div * third);
     // neighbour cells: normal stress along the shared face's normal
     T sL, sR, sF, sB, sD, sU;
     {   // cell (i-1, j, k): faces vx[F-sy], vx[F]; vy[F-sy], vy[F-sy+1]; vz[F-sy], vz[F-sy+sz]
         const T a = (vx0 - vxm) * hx0, b = (vyxY - vyx_) * hy1, c = (vzxZ - vzx_) * hz1;
-        sL = two * eta_at(L, L.ec, u - sy) * (a - (a + b + c) * third);
+        sL = two * E(1) * (a - (a + b + c) * third);
     }
     {   // cell (i+1, j, k)
         const T a = (vxXX - vxX) * hx2, b = (vyXY - vyX) * hy1, c = (vzXZ - vzX) * hz1;
-        sR = two * eta_at(L, L.ec, u + sy) * (a - (a + b + c) * third);
+        sR = two * E(2) * (a - (a + b + c) * third);
     }
     {   // cell (i, j-1, k)
         const T a = (vxXy - vxy_) * hx1, b = (vy0 - vym) * hy0, c = (vzyZ - vzy_) * hz1;
-        sF = two * eta_at(L, L.ec, u - 1) * (b - (a + b + c) * third);
+        sF = two * E(3) * (b - (a + b + c) * third);
     }
     {   // cell (i, j+1, k)
         const T a = (vxXY - vxY) * hx1, b = (vyYY - vyY) * hy2, c = (vzYZ - vzY) * hz1;
-        sB = two * eta_at(L, L.ec, u + 1) * (b - (a + b + c) * third);
+        sB = two * E(4) * (b - (a + b + c) * third);
     }
     {   // cell (i, j, k-1)
         const T a = (vxXz - vxz_) * hx1, b = (vyYz - vyz_) * hy1, c = (vz0 - vzm) * hz0;
-        sD = two * eta_at(L, L.ec, u - sz) * (c - (a + b + c) * third);
+        sD = two * E(5) * (c - (a + b + c) * third);
     }
     {   // cell (i, j, k+1)
         const T a = (vxXZ - vxZ) * hx1, b = (vyYZ - vyZ) * hy1, c = (vzZZ - vzZ) * hz2;
-        sU = two * eta_at(L, L.ec, u + sz) * (c - (a + b + c) * third);
+        sU = two * E(6) * (c - (a + b + c) * third);
     }
     // edge shear stresses (sxy, sxz, syz at the cell's twelve edges)
-    const T ex0 = L.ax.ihe[i - 1], ex1 = L.ax.ihe[i], ey0 = L.ay.ihe[j - 1], ey1 = L.ay.ihe[j];
-    const T ez0 = L.az.ihe[k - 1], ez1 = L.az.ihe[k];
-    const T xy00 = two * eta_at(L, L.exy, F) * ((vx0 - vxy_) * ey0 + (vy0 - vyx_) * ex0);
-    const T xy01 = two * eta_at(L, L.exy, F + 1) * ((vxY - vx0) * ey1 + (vyY - vyxY) * ex0);
-    const T xy10 = two * eta_at(L, L.exy, F + sy) * ((vxX - vxXy) * ey0 + (vyX - vy0) * ex1);
-    const T xy11 = two * eta_at(L, L.exy, F + sy + 1) * ((vxXY - vxX) * ey1 + (vyXY - vyY) * ex1);
-    const T xz00 = two * eta_at(L, L.exz, F) * ((vx0 - vxz_) * ez0 + (vz0 - vzx_) * ex0);
-    const T xz01 = two * eta_at(L, L.exz, F + sz) * ((vxZ - vx0) * ez1 + (vzZ - vzxZ) * ex0);
-    const T xz10 = two * eta_at(L, L.exz, F + sy) * ((vxX - vxXz) * ez0 + (vzX - vz0) * ex1);
-    const T xz11 = two * eta_at(L, L.exz, F + sy + sz) * ((vxXZ - vxX) * ez1 + (vzXZ - vzZ) * ex1);
-    const T yz00 = two * eta_at(L, L.eyz, F) * ((vy0 - vyz_) * ez0 + (vz0 - vzy_) * ey0);
-    const T yz01 = two * eta_at(L, L.eyz, F + sz) * ((vyZ - vy0) * ez1 + (vzZ - vzyZ) * ey0);
-    const T yz10 = two * eta_at(L, L.eyz, F + 1) * ((vyY - vyYz) * ez0 + (vzY - vz0) * ey1);
-    const T yz11 = two * eta_at(L, L.eyz, F + 1 + sz) * ((vyYZ - vyY) * ez1 + (vzYZ - vzZ) * ey1);
-    const T *pp = x.p + u;
-    const T p0 = __ldg(pp), pL = __ldg(pp - sy), pR = __ldg(pp + sy), pF = __ldg(pp - 1),
-            pB = __ldg(pp + 1);
-    const T pD = __ldg(pp - sz), pU = __ldg(pp + sz);
-    const T cx0 = L.ax.ihc[i - 1], cx1 = L.ax.ihc[i], cy0 = L.ay.ihc[j - 1], cy1 = L.ay.ihc[j];
-    const T cz0 = L.az.ihc[k - 1], cz1 = L.az.ihc[k];
-    const T wx = L.ax.ihv[i - 1], wy = L.ay.ihv[j - 1], wz = L.az.ihv[k - 1];
+    const T ex0 = AX.ihe[i - 1], ex1 = AX.ihe[i], ey0 = AY.ihe[j - 1], ey1 = AY.ihe[j];
+    const T ez0 = AZ.ihe[k - 1], ez1 = AZ.ihe[k];
+    const T xy00 = two * E(7) * ((vx0 - vxy_) * ey0 + (vy0 - vyx_) * ex0);
+    const T xy01 = two * E(8) * ((vxY - vx0) * ey1 + (vyY - vyxY) * ex0);
+    const T xy10 = two * E(9) * ((vxX - vxXy) * ey0 + (vyX - vy0) * ex1);
+    const T xy11 = two * E(10) * ((vxXY - vxX) * ey1 + (vyXY - vyY) * ex1);
+    const T xz00 = two * E(11) * ((vx0 - vxz_) * ez0 + (vz0 - vzx_) * ex0);
+    const T xz01 = two * E(12) * ((vxZ - vx0) * ez1 + (vzZ - vzxZ) * ex0);
+    const T xz10 = two * E(13) * ((vxX - vxXz) * ez0 + (vzX - vz0) * ex1);
+    const T xz11 = two * E(14) * ((vxXZ - vxX) * ez1 + (vzXZ - vzZ) * ex1);
+    const T yz00 = two * E(15) * ((vy0 - vyz_) * ez0 + (vz0 - vzy_) * ey0);
+    const T yz01 = two * E(16) * ((vyZ - vy0) * ez1 + (vzZ - vzyZ) * ey0);
+    const T yz10 = two * E(17) * ((vyY - vyYz) * ez0 + (vzY - vz0) * ey1);
+    const T yz11 = two * E(18) * ((vyYZ - vyY) * ez1 + (vzYZ - vzZ) * ey1);
+    const T p0 = PR(0), pL = PR(1), pR = PR(2), pF = PR(3), pB = PR(4), pD = PR(5), pU = PR(6);
+    const T cx0 = AX.ihc[i - 1], cx1 = AX.ihc[i], cy0 = AY.ihc[j - 1], cy1 = AY.ihc[j];
+    const T cz0 = AZ.ihc[k - 1], cz1 = AZ.ihc[k];
+    const T wx = AX.ihv[i - 1], wy = AY.ihv[j - 1], wz = AZ.ihv[k - 1];
     ax[0] = (s0 - sL) * cx0 + (xy01 - xy00) * wy + (xz01 - xz00) * wz - (p0 - pL) * cx0;
     ax[1] = (sR - s0) * cx1 + (xy11 - xy10) * wy + (xz11 - xz10) * wz - (pR - p0) * cx1;
     ax[2] = (s1 - sF) * cy0 + (xy10 - xy00) * wx + (yz01 - yz00) * wz - (p0 - pF) * cy0;
     ax[3] = (sB - s1) * cy1 + (xy11 - xy01) * wx + (yz11 - yz10) * wz - (pB - p0) * cy1;
     ax[4] = (s2 - sD) * cz0 + (xz10 - xz00) * wx + (yz10 - yz00) * wy - (p0 - pD) * cz0;
     ax[5] = (sU - s2) * cz1 + (xz11 - xz01) * wx + (yz11 - yz01) * wy - (pU - p0) * cz1;
+    if (kDiag) {
+        const T t43 = (T)(4.0 / 3.0);
+        const T eC = E(0), eL = E(1), eR = E(2), eF = E(3), eB = E(4), eD = E(5), eU = E(6);
+        const T nxy00 = E(7), nxy01 = E(8), nxy10 = E(9), nxy11 = E(10);
+        const T nxz00 = E(11), nxz01 = E(12), nxz10 = E(13), nxz11 = E(14);
+        const T nyz00 = E(15), nyz01 = E(16), nyz10 = E(17), nyz11 = E(18);
+        d[0] = -(cx0 * t43 * (eC * hx1 + eL * hx0) + wy * two * (nxy01 * ey1 + nxy00 * ey0) + wz * two * (nxz01 * ez1 + nxz00 * ez0));
+        d[1] = -(cx1 * t43 * (eR * hx2 + eC * hx1) + wy * two * (nxy11 * ey1 + nxy10 * ey0) + wz * two * (nxz11 * ez1 + nxz10 * ez0));
+        d[2] = -(cy0 * t43 * (eC * hy1 + eF * hy0) + wx * two * (nxy10 * ex1 + nxy00 * ex0) + wz * two * (nyz01 * ez1 + nyz00 * ez0));
+        d[3] = -(cy1 * t43 * (eB * hy2 + eC * hy1) + wx * two * (nxy11 * ex1 + nxy01 * ex0) + wz * two * (nyz11 * ez1 + nyz10 * ez0));
+        d[4] = -(cz0 * t43 * (eC * hz1 + eD * hz0) + wx * two * (nxz10 * ex1 + nxz00 * ex0) + wy * two * (nyz10 * ey1 + nyz00 * ey0));
+        d[5] = -(cz1 * t43 * (eU * hz2 + eC * hz1) + wx * two * (nxz11 * ex1 + nxz01 * ex0) + wy * two * (nyz11 * ey1 + nyz01 * ey0));
+    }
+}
+
+// The same on a level's own fields.
+template <typename T>
+__device__ __forceinline__ void cell_rows(const LevelView<T> &L, const Fields<T, T> &x, int i, int j, int k,
+                                          const int fi[6], T ax[6], T &div)
+{
+    cell_rows<T, false>(L.ax, L.ay, L.az, L.ny, L.nx * L.ny, x, i, j, k, fi[0], LevelEta<T>{L, fi[0]}, LoadConst{}, ax,
+                        div, (T *)nullptr);
 }
 
 // Cell of thread t in colour col (cells with (i + j + k) of one parity), or
@@ -463,6 +478,66 @@ __device__ __forceinline__ void cell_faces(const LevelView<T> &L, int i, int j, 
     fi[3] = P2IDX(L, i - 1, j, k - 1);
     fi[4] = fi[0];
     fi[5] = P2IDX(L, i - 1, j - 1, k);
+}
+
+// ---------------------------------------------------------------------------
+// One colour pass of the cell-block smoother with a diagonal velocity block
+// (diagonal Vanka / SCGS) over the cells with (i+j+k)&1 == col.  Each cell
+// corrects its six face velocities and its pressure together with the velocity
+// block replaced by its diagonal:
+//   d_v dv_v + g_v dp = r_v,  sum_v c_v dv_v = r_p.
+// Every cell of the colour reads the state from before the pass: velocities
+// are read from vin and written to vout (each face belongs to exactly one
+// cell of each colour), the pressure is updated in place (a cell's pressure is
+// read only by its own face rows among the cells of one colour).  Residuals
+// and diagonals come from one set of loads (cell_rows); evaluated row by row
+// the FP32 pass took 133 us at 129^3, now 96 us, and 17 us, now 12 us, at 36^3.
+template <typename T>
+__device__ __forceinline__ void vanka_item(const LevelView<T> &L, T *P, const Vec4<T> &vin, const Vec4<T> &vout,
+                                           const Vec4<T> &b, T omega, int col, long t)
+{
+    int i, j, k;
+    if (!colour_cell(L, col, t, i, j, k)) return;
+    Fields<T, T> x{P, vin.c[1], vin.c[2], vin.c[3]};
+    const int u = P2IDX(L, i, j, k);
+    const bool pbc = (L.bcm[u] & BC_P) != 0;
+    int fi[6];
+    const int fc[6] = {1, 1, 2, 2, 3, 3};
+    cell_faces(L, i, j, k, fi);
+    bool act[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) act[q] = !(L.bcm[fi[q]] & (1 << fc[q]));
+    T ax[6], d[6], div;
+    cell_rows<T, true>(L.ax, L.ay, L.az, L.ny, L.nx * L.ny, x, i, j, k, fi[0], LevelEta<T>{L, fi[0]}, LoadConst{}, ax,
+                       div, d);
+    const T g[6] = {-L.ax.ihc[i - 1], L.ax.ihc[i], -L.ay.ihc[j - 1], L.ay.ihc[j], -L.az.ihc[k - 1], L.az.ihc[k]};
+    const T hx = L.ax.ih[i], hy = L.ay.ih[j], hz = L.az.ih[k];
+    const T cc[6] = {-hx, hx, -hy, hy, -hz, hz};
+    T num = 0, den = 0, r[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+        r[q] = act[q] ? b.c[fc[q]][fi[q]] - ax[q] : (T)0;
+        if (act[q]) {
+            num += cc[q] * r[q] / d[q];
+            den += cc[q] * g[q] / d[q];
+        }
+    }
+    T dp = 0;
+    if (!pbc && den != (T)0) {
+        dp = (num - (b.c[0][u] - div)) / den;
+        P[u] += omega * dp;
+    }
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+        if (act[q] && d[q] != (T)0)
+            vout.c[fc[q]][fi[q]] = vin.c[fc[q]][fi[q]] + omega * (r[q] - g[q] * dp) / d[q];
+}
+template <typename T>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 3) k_vanka(LevelView<T> L, T *P, Vec4<T> vin, Vec4<T> vout, Vec4<T> b, T omega,
+                                               int col)
+{
+    pdl_enter();
+    vanka_item(L, P, vin, vout, b, omega, col, (long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -575,12 +650,6 @@ __global__ void __launch_bounds__(128) k_vanka_fast(LevelView<T> L, T *P, Vec4<T
 // same update as k_vanka_full up to rounding, without building and
 // eliminating the 6x6 block on every sweep.
 constexpr int kBlkEntries = 22;
-// minimum resident blocks per SM asked of the compiler for k_vanka_stored
-// (FP32 cycle; the FP64 cycle's kernel needs more registers)
-#ifndef P2_STORED_MIN_BLOCKS
-#define P2_STORED_MIN_BLOCKS 7
-#endif
-
 // packed upper-triangle index of (a, c), a <= c
 __host__ __device__ constexpr int tri_index(int a, int c) { return a * 6 - a * (a - 1) / 2 + (c - a); }
 
@@ -722,8 +791,14 @@ __device__ __forceinline__ void vanka_stored_item(const LevelView<T> &L, T *P, c
     for (int q = 0; q < 6; q++)
         if (act[q]) vout.c[fc[q]][fi[q]] = vin.c[fc[q]][fi[q]] + omega * (y1[q] - dp * y2[q]);
 }
+// Latency-bound: what counts is how many of a cell's about 70 loads are in
+// flight.  FP32: 128 registers, with the viscosities and pressures loaded ahead
+// (cell_rows): 72 / 16.4 / 10.3 / 8.8 us a pass on the levels of 129^3 where 72
+// registers with seven blocks an SM took 74 / 20.7 / 12.4 / 12.3 us.  FP64: 168
+// registers, loads where they are used: 176 us against 199 us, and 205 us with
+// the loads ahead.
 template <typename T>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? P2_STORED_MIN_BLOCKS : 3) k_vanka_stored(
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 3) k_vanka_stored(
     LevelView<T> L, T *P, Vec4<T> vin, Vec4<T> vout, Vec4<T> b, T omega, int col,
     const factor_t<T> *__restrict__ blk, long stride)
 {

@@ -1001,7 +1001,7 @@ void Solver::smoother_pass(int l, const LevelView<T> &V, T *P, Vec4<T> &vin, Vec
     }
     case 2: pdl_launch(st, nblk(cells, 128), 128, k_vanka_full<T>, V, P, vin, vout, b, om, col); break;
     case 3: pdl_launch(st, nblk(cells, 128), 128, k_vanka_fast<T>, V, P, vin, vout, b, om, col); break;
-    default: pdl_launch(st, nblk(cells), kThreads, k_vanka<T>, V, P, vin, vout, b, om, col); break;
+    default: pdl_launch(st, nblk(cells, 128), 128, k_vanka<T>, V, P, vin, vout, b, om, col); break;
     }
 }
 
