@@ -27,8 +27,8 @@ struct Basis {
     const double2 *v[kMaxBasis];
 };
 
-// hcol: h_0 .. h_{k}, then these
-enum { HC_SIGMA = kMaxBasis, HC_QQ, HC_WW, HC_LEN };
+// hcol: h_0 .. h_{k}, then these (HC_ERROR: set by a smoother whose barrier ran out of time)
+enum { HC_SIGMA = kMaxBasis, HC_QQ, HC_WW, HC_ERROR, HC_LEN };
 
 inline unsigned basis_blocks(long n2, int u)
 {

@@ -27,6 +27,7 @@
 #include "p2_sweep.cuh"
 #include "p2_zmarch.cuh"
 #include "p2_coarse.cuh"
+#include "p2_resident.cuh"
 
 namespace p2 {
 
@@ -231,6 +232,7 @@ Solver::Solver(int device) : dev(device)
         P2_CUDA_TRY(cudaStreamCreateWithPriority(&st_lu, cudaStreamNonBlocking, hi));
     }
     P2_CUDA_TRY(cudaEventCreateWithFlags(&ev_lu, cudaEventDisableTiming));
+    P2_CUDA_TRY(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
     for (int i = 0; i < 8; i++) P2_CUDA_TRY(cudaEventCreate(&ev[i]));
 }
 
@@ -551,6 +553,7 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
             if (order.empty()) order.push_back(0);
             Lv.sw_order = upload(arena, order);
         }
+        build_resident(Lv);
         Lv.h_bcm = m;
         Lv.bcm = upload(arena, m);
         Lv.bu = upload(arena, bu);
@@ -561,6 +564,70 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
     }
     allocate_work();
     bc_ready = true;
+}
+
+// Resident sweeps (p2_resident.cuh): whether the level's cells fit, in which
+// form, and the boundary rows that follow each cell's unknowns.
+void Solver::build_resident(Level &Lv)
+{
+    const long half = Lv.ny / 2, slots = (long)(Lv.nx - 1) * (Lv.nz - 1) * half;
+    Lv.res_mode = 0;
+    auto per_block = [&](long blocks) { return (int)(((slots + blocks - 1) / blocks + 31) / 32 * 32); };
+    if (per_block(kResCluster) <= kResSlots) {
+        Lv.res_mode = 1;
+        Lv.res_blocks = kResCluster;
+    } else if (per_block(sm_count) <= kResSlots) {
+        Lv.res_mode = 2;
+        Lv.res_blocks = (int)((slots + per_block(sm_count) - 1) / per_block(sm_count));
+    } else {
+        return;
+    }
+    Lv.res_slots = per_block(Lv.res_blocks);
+    // two passes over the rows: count per colour and slot, then place
+    std::vector<int> ptr(2 * slots + 1, 0), at;
+    std::vector<int4> dep;
+    for (int pass = 0; pass < 2; pass++) {
+        for (size_t q = 0; q < Lv.h_bu.size(); q++) {
+            const int t = Lv.h_rt[q];
+            if (t < 0) continue;
+            const float rk = (float)Lv.h_rk[q];
+            const int c = t & 3, v = t >> 2;
+            const int j = v % Lv.ny, i = (v / Lv.ny) % Lv.nx, k = v / (Lv.nx * Lv.ny);
+            int kbits;
+            std::memcpy(&kbits, &rk, sizeof kbits);
+            auto follow = [&](int ci, int cj, int ck, int face) {
+                // a target that is no cell's unknown keeps its value through the sweeps
+                if (ci < 1 || cj < 1 || ck < 1 || ci >= Lv.nx || cj >= Lv.ny || ck >= Lv.nz) return;
+                const long slot = ((ci + cj + ck) & 1) * slots + ((long)(ck - 1) * (Lv.nx - 1) + (ci - 1)) * half + (cj - 1) / 2;
+                if (pass == 0) ptr[slot + 1]++;
+                else dep[at[slot]++] = make_int4(face, Lv.h_bu[q], (int)q, kbits);
+            };
+            // the cells on both sides of a face (one of each colour), or the pressure's own cell
+            if (c == 0) follow(i, j, k, 6);
+            else if (c == 1) { follow(i, j + 1, k + 1, 1); follow(i + 1, j + 1, k + 1, 0); }
+            else if (c == 2) { follow(i + 1, j, k + 1, 3); follow(i + 1, j + 1, k + 1, 2); }
+            else { follow(i + 1, j + 1, k, 5); follow(i + 1, j + 1, k + 1, 4); }
+        }
+        if (pass == 0) {
+            for (long e = 0; e < 2 * slots; e++) ptr[e + 1] += ptr[e];
+            at.assign(ptr.begin(), ptr.end() - 1);
+            dep.resize(ptr[2 * slots]);
+        }
+    }
+    Lv.res_cap = 0;
+    for (long s0 = 0; s0 < slots; s0 += Lv.res_slots) {
+        const long s1 = std::min(s0 + Lv.res_slots, slots);
+        Lv.res_cap = std::max(Lv.res_cap, ptr[s1] - ptr[s0] + ptr[slots + s1] - ptr[slots + s0]);
+    }
+    Lv.res_cap = (Lv.res_cap + 1) / 2 * 2;
+    const size_t most = std::max(res_smem<double, true>(2 * Lv.res_slots, Lv.tabstride, Lv.res_cap),
+                                 res_smem<float, true>(2 * Lv.res_slots, Lv.tabstride, Lv.res_cap));
+    if (most > kResSmemMax) {
+        Lv.res_mode = 0;
+        return;
+    }
+    Lv.res_ptr = upload(arena, ptr);
+    Lv.res_dep = upload(arena, dep);
 }
 
 void Solver::allocate_work()
@@ -636,6 +703,7 @@ void Solver::allocate_work()
     hcol = (double *)arena.alloc(sizeof(double) * HC_LEN);
     partial = (double *)arena.alloc(sizeof(double) * kRedBlocks * kMaxBasis);
     dticket = (unsigned *)arena.alloc(sizeof(unsigned) * 4);
+    res_count = (unsigned *)arena.alloc(sizeof(unsigned) * 4);
     {
         long maxc = 1;
         for (int l = 1; l < nl; l++) maxc = std::max<long>(maxc, L[l].n);
@@ -1084,12 +1152,58 @@ void Solver::sweep_fused(int l, const LevelView<T> &V, Vec4<T> &xin, Vec4<T> &xo
 #endif
 }
 
+// All sweeps of a small level in one launch (res_mode 1: one cluster, 2: a
+// cooperative grid).
+template <typename T, bool kFull>
+void Solver::smooth_resident(int l, int sweeps)
+{
+    Level &Lv = L[l];
+    LevelView<T> V = view<T>(l, false);
+    const int threads = 2 * Lv.res_slots, mx = Lv.tabstride;
+    const size_t smem = res_smem<T, kFull>(threads, mx, Lv.res_cap);
+    const ResidentBC R{Lv.nbc, Lv.bu, Lv.bt, Lv.bnext, Lv.bk, Lv.res_ptr, Lv.res_dep, Lv.res_cap};
+    const T *tab = std::is_same<T, double>::value ? (const T *)Lv.tabd : (const T *)Lv.tabf;
+    const bool cluster = Lv.res_mode == 1;
+    auto kern = cluster ? k_smooth_resident<T, kFull, true> : k_smooth_resident<T, kFull, false>;
+    // the same value from every thread: the attribute belongs to the function, not to this context
+    P2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemMax));
+    if (cluster) P2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(Lv.res_blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (cluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = Lv.res_blocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
+    } else {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.numAttrs = 1;
+    }
+    P2_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, V, vx_of<T>(Lv, 0), vx_of<T>(Lv, 1), b_of<T>(Lv), (T)prm.omega, 2 * sweeps,
+                                   (const factor_t<T> *)Lv.blk, Lv.blk_stride, R, mx, tab,
+                                   GridBarrier{res_count, hcol + HC_ERROR}));
+    P2_COUNT_LAUNCH();
+}
+
 template <typename T>
 void Solver::smooth(int l, int sweeps)
 {
     Level &Lv = L[l];
     LevelView<T> V = view<T>(l, false);
     Vec4<T> &x = vx_of<T>(Lv, 0), &y = vx_of<T>(Lv, 1), &b = b_of<T>(Lv);
+    if (sweeps > 0 && Lv.res_mode && (prm.smoother == 0 || prm.smoother == 1)) {
+        if (prm.smoother == 1) smooth_resident<T, true>(l, sweeps);
+        else smooth_resident<T, false>(l, sweeps);
+        return;
+    }
     bc_set<T>(l, x, b);
     if (sweeps <= 0) return;
     // colour 0 reads velocities from x and writes y, colour 1 goes back; the
@@ -1362,6 +1476,12 @@ p2_solve_info Solver::solve()
             P2_CUDA_TRY(cudaMemcpyAsync(hc, hcol, sizeof(double) * HC_LEN, cudaMemcpyDeviceToHost, st));
             P2_CUDA_TRY(cudaStreamSynchronize(st));
             it++;
+            if (hc[HC_ERROR] != 0) {
+                P2_CUDA_TRY(cudaMemsetAsync(res_count, 0, sizeof(unsigned) * 4, st));
+                P2_CUDA_TRY(cudaMemsetAsync(hcol + HC_ERROR, 0, sizeof(double), st));
+                P2_CUDA_TRY(cudaStreamSynchronize(st));
+                throw Error(P2_ERR_CUDA, "a grid barrier of the smoother ran out of time");
+            }
             const double sigma = hc[HC_SIGMA], wn2 = hc[HC_WW];
             // a direction without a positive norm, or not a number
             if (!(hc[HC_QQ] > 0) || !std::isfinite(wn2) || !std::isfinite(hc[HC_QQ])) { bad = true; break; }

@@ -49,6 +49,10 @@ struct Level {
     // within one node; the rows by node (first row per node, row order)
     bool fuse_ok = false;
     int *sw_first = nullptr, *sw_order = nullptr;
+    // resident sweeps (k_smooth_resident): 0 none, 1 one cluster, 2 cooperative grid
+    int res_mode = 0, res_blocks = 0, res_slots = 0, res_cap = 0;
+    int *res_ptr = nullptr;
+    int4 *res_dep = nullptr;
     // boundary rows sorted by copy-chain depth
     int nbc = 0;
     std::vector<int> bc_groups;
@@ -206,6 +210,11 @@ class Solver {
     void bc_set(int l, Vec4<T> &x, Vec4<T> &b);
     template <typename T>
     void smooth(int l, int sweeps);
+    template <typename T, bool kFull>
+    void smooth_resident(int l, int sweeps);
+    void build_resident(Level &Lv);
+    int sm_count = 0;
+    unsigned *res_count = nullptr;  // grid barrier counters of the resident sweeps
     template <typename T>
     void smoother_pass(int l, const LevelView<T> &V, T *P, Vec4<T> &vin, Vec4<T> &vout, Vec4<T> &b, int col);
     bool use_fused(int l) const;
