@@ -355,6 +355,9 @@ struct AxisMap {
     // inverse lists: coarse index I -> fine (idx, weight)
     const int *ptr, *idx;
     const double *w;
+    // the same lists padded to a fixed number of entries per coarse index (restriction only)
+    const int *pidx;
+    const double *pw;
 };
 // type per axis: 0 node-located, 1 mid-located, 2 pressure cell centre
 struct TransferView {

@@ -20,37 +20,105 @@ __device__ __forceinline__ S to_factor(double v) { return (S)v; }
 constexpr int kThreads = 256;
 
 // ---------------------------------------------------------------------------
+// The three momentum rows at node (i, j, k), 1 <= i <= nx-2 and so on, from
+// shared stresses: the upper cell's three normal stresses, the one along the
+// row's axis of its lower x, y and z neighbours, three edges of each
+// orientation; every velocity, viscosity and pressure loaded once.  The same
+// terms as row_vx / row_vy / row_vz up to rounding (the deviatoric third is a
+// multiplication by 1/3).
+template <typename T, typename S>
+__device__ __forceinline__ void node_rows(const LevelView<T> &L, const Fields<T, S> &x, int i, int j, int k, T r[3])
+{
+    const int sy = L.ny, sz = L.nx * L.ny, u = P2IDX(L, i, j, k);
+    const S *vx = x.vx + u, *vy = x.vy + u, *vz = x.vz + u, *pp = x.p + u + sz + sy + 1;
+    auto V = [](const S *q) { return (T)__ldg(q); };
+    const T vx0 = V(vx), vxX = V(vx + sy), vxm = V(vx - sy), vxY = V(vx + 1), vxy_ = V(vx - 1), vxZ = V(vx + sz),
+            vxz_ = V(vx - sz), vxXy = V(vx + sy - 1), vxXz = V(vx + sy - sz);
+    const T vy0 = V(vy), vyY = V(vy + 1), vym = V(vy - 1), vyX = V(vy + sy), vyx_ = V(vy - sy), vyZ = V(vy + sz),
+            vyz_ = V(vy - sz), vyYx = V(vy + 1 - sy), vyYz = V(vy + 1 - sz);
+    const T vz0 = V(vz), vzZ = V(vz + sz), vzm = V(vz - sz), vzX = V(vz + sy), vzx_ = V(vz - sy), vzY = V(vz + 1),
+            vzy_ = V(vz - 1), vzZx = V(vz + sz - sy), vzZy = V(vz + sz - 1);
+    const T pA = V(pp), pL = V(pp - sy), pF = V(pp - 1), pD = V(pp - sz);
+    const T third = (T)(1.0 / 3.0), two = (T)2.0;
+    const T hx0 = L.ax.ih[i], hx1 = L.ax.ih[i + 1], hy0 = L.ay.ih[j], hy1 = L.ay.ih[j + 1], hz0 = L.az.ih[k],
+            hz1 = L.az.ih[k + 1];
+    const int c = u + sz + sy + 1;
+    T sAx, sAy, sAz, sL, sF, sD;
+    {
+        const T a = (vxX - vx0) * hx1, b = (vyY - vy0) * hy1, d = (vzZ - vz0) * hz1, m = (a + b + d) * third;
+        const T E = two * eta_at(L, L.ec, c);
+        sAx = E * (a - m);
+        sAy = E * (b - m);
+        sAz = E * (d - m);
+    }
+    {
+        const T a = (vx0 - vxm) * hx0, b = (vyYx - vyx_) * hy1, d = (vzZx - vzx_) * hz1;
+        sL = two * eta_at(L, L.ec, c - sy) * (a - (a + b + d) * third);
+    }
+    {
+        const T a = (vxXy - vxy_) * hx1, b = (vy0 - vym) * hy0, d = (vzZy - vzy_) * hz1;
+        sF = two * eta_at(L, L.ec, c - 1) * (b - (a + b + d) * third);
+    }
+    {
+        const T a = (vxXz - vxz_) * hx1, b = (vyYz - vyz_) * hy1, d = (vz0 - vzm) * hz0;
+        sD = two * eta_at(L, L.ec, c - sz) * (d - (a + b + d) * third);
+    }
+    const T ex0 = L.ax.ihe[i], ex1 = L.ax.ihe[i + 1], ey0 = L.ay.ihe[j], ey1 = L.ay.ihe[j + 1], ez0 = L.az.ihe[k],
+            ez1 = L.az.ihe[k + 1];
+    const T xy0 = two * eta_at(L, L.exy, u) * ((vx0 - vxy_) * ey0 + (vy0 - vyx_) * ex0);
+    const T xyY = two * eta_at(L, L.exy, u + 1) * ((vxY - vx0) * ey1 + (vyY - vyYx) * ex0);
+    const T xyX = two * eta_at(L, L.exy, u + sy) * ((vxX - vxXy) * ey0 + (vyX - vy0) * ex1);
+    const T xz0 = two * eta_at(L, L.exz, u) * ((vx0 - vxz_) * ez0 + (vz0 - vzx_) * ex0);
+    const T xzZ = two * eta_at(L, L.exz, u + sz) * ((vxZ - vx0) * ez1 + (vzZ - vzZx) * ex0);
+    const T xzX = two * eta_at(L, L.exz, u + sy) * ((vxX - vxXz) * ez0 + (vzX - vz0) * ex1);
+    const T yz0 = two * eta_at(L, L.eyz, u) * ((vy0 - vyz_) * ez0 + (vz0 - vzy_) * ey0);
+    const T yzZ = two * eta_at(L, L.eyz, u + sz) * ((vyZ - vy0) * ez1 + (vzZ - vzZy) * ey0);
+    const T yzY = two * eta_at(L, L.eyz, u + 1) * ((vyY - vyYz) * ez0 + (vzY - vz0) * ey1);
+    const T cx = L.ax.ihc[i], cy = L.ay.ihc[j], cz = L.az.ihc[k], wx = L.ax.ihv[i], wy = L.ay.ihv[j], wz = L.az.ihv[k];
+    r[0] = (sAx - sL) * cx + (xyY - xy0) * wy + (xzZ - xz0) * wz - (pA - pL) * cx;
+    r[1] = (sAy - sF) * cy + (xyX - xy0) * wx + (yzZ - yz0) * wz - (pA - pF) * cy;
+    r[2] = (sAz - sD) * cz + (xzX - xz0) * wx + (yzY - yz0) * wy - (pA - pD) * cz;
+}
+
 // Rows: out = b - A x (mode 0) or out = A x (mode 1) on every non-boundary
 // row; boundary rows and non-unknown positions get 0 here (boundary rows are
 // written by k_bc_rows).  Optionally also writes a float copy (the FP32
-// right-hand side of the mixed-precision V-cycle).
+// right-hand side of the mixed-precision V-cycle) or a copy of x (the outer
+// loop's stored correction).  All four rows of a node in one thread from one
+// set of loads: evaluated one after the other, with a store between them, each
+// row loaded and derived its stresses anew.  Waits for loads: 8 (FP32) or 4
+// (FP64) blocks of 128 threads an SM measured best of 5 .. 10 and 3 .. 6.  257^3:
+// q = A c from FP32 with its copy 0.99 ms (and 0.17 ms for the copy) -> 0.72 ms,
+// FP32 residual 0.66 -> 0.60 ms, 67^3 26 -> 20 us; the FP64 residual, once per
+// restart, 1.08 -> 1.29 ms.
+constexpr int kRowsThreads = 128;
 template <typename T, typename S>
-__device__ __forceinline__ void rows_item(const LevelView<T> &L, const Fields<T, S> &x, const Vec4<T> &b,
-                                          const Vec4<T> &out, const Vec4<float> &out32, int mode, int u)
-{
-    if (u >= L.n) return;
-    int j = u % L.ny, i = (u / L.ny) % L.nx, k = u / (L.nx * L.ny);
-    uint8_t m = L.bcm[u];
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        T v = 0;
-        if (valid_pos(c, i, j, k, L.nx, L.ny, L.nz) && !(m & (1 << c))) {
-            T ax;
-            if (c == 0) ax = row_p(L, x, i, j, k);
-            else if (c == 1) ax = row_vx(L, x, i, j, k, (T *)nullptr);
-            else if (c == 2) ax = row_vy(L, x, i, j, k, (T *)nullptr);
-            else ax = row_vz(L, x, i, j, k, (T *)nullptr);
-            v = mode == 0 ? b.c[c][u] - ax : ax;
-        }
-        out.c[c][u] = v;
-        if (out32.c[0]) out32.c[c][u] = (float)v;
-    }
-}
-template <typename T, typename S>
-__global__ void k_rows(LevelView<T> L, Fields<T, S> x, Vec4<T> b, Vec4<T> out, Vec4<float> out32, int mode)
+__global__ void __launch_bounds__(kRowsThreads, sizeof(T) == 4 ? 8 : 4) k_rows(LevelView<T> L, Fields<T, S> x,
+                                                                             Vec4<T> b, Vec4<T> out,
+                                                                             Vec4<float> out32, Vec4<S> copy, int mode)
 {
     pdl_enter();
-    rows_item(L, x, b, out, out32, mode, blockIdx.x * blockDim.x + threadIdx.x);
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= L.n) return;
+    const int j = u % L.ny, i = (u / L.ny) % L.nx, k = u / (L.nx * L.ny);
+    const uint8_t m = L.bcm[u];
+    T v[4] = {0, 0, 0, 0}, r[3];
+    if (i > 0 && j > 0 && k > 0) {
+        if (!(m & BC_P)) v[0] = row_p(L, x, i, j, k);
+        if (i < L.nx - 1 && j < L.ny - 1 && k < L.nz - 1 && (m & (BC_VX | BC_VY | BC_VZ)) != (BC_VX | BC_VY | BC_VZ)) {
+            node_rows(L, x, i, j, k, r);
+#pragma unroll
+            for (int c = 1; c < 4; c++) v[c] = r[c - 1];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const bool row = valid_pos(c, i, j, k, L.nx, L.ny, L.nz) && !(m & (1 << c));
+        const T w = !row ? (T)0 : (mode == 0 ? b.c[c][u] - v[c] : v[c]);
+        out.c[c][u] = w;
+        if (out32.c[0]) out32.c[c][u] = (float)w;
+        if (copy.c[0]) copy.c[c][u] = (c == 0 ? x.p : c == 1 ? x.vx : c == 2 ? x.vy : x.vz)[u];
+    }
 }
 
 // Boundary rows x_u = b_u + koef * x_t: residual (mode 0) b_u + koef x_t - x_u,
@@ -827,109 +895,147 @@ __device__ __forceinline__ AxisMap pick_map(const AxisMap (&m)[3], int type)
 
 // Restriction (vprestrict, move3mgNew.c:3965-4353): b_c = sum_f w r_f / sum_f w
 // over the non-boundary fine rows (pressure residuals scaled by eta_f/eta_c,
-// 4308), for non-boundary coarse rows (0 otherwise); x_c = 0 (4351).  One
-// thread per (coarse node, component), components in consecutive blocks of
-// nodes.  Fused with the first half of the coarse
-// right-hand-side compatibility shift: every block adds its volume-weighted
-// continuity rows into partial[block]; the last block to finish (ticket
-// counter, reset by that block) sums the partials in block order and writes
-// sums[0] = sum of vol * b_P and sums[1] = vol_total (fixed per level).
-constexpr int kRestrictList = 5;  // longest inverse list of one axis (host-checked)
+// 4308), for non-boundary coarse rows (0 otherwise); x_c = 0 (4351).  The
+// residual is 0 on boundary rows, so the numerator needs no mask; the weights'
+// sums without them are fixed by the tables (k_restrict_weights).  A block
+// takes 256 / kSplit consecutive (component, coarse node) pairs, components
+// outermost, and its kSplit groups of threads take the entries of the z lists
+// in turn.  Without the mask loads and the weight sums 257^3 -> 131^3 takes 0.63
+// ms (0.94 with them, 0.05 of the HBM rate: bound by its gathers' instructions),
+// 20^3 -> 12^3 14.5 us with four threads a pair (23.5 us).  Fused with the first half of the coarse
+// right-hand-side compatibility shift: every block with pressure rows adds its
+// volume-weighted continuity rows into partial[block]; the last of them to
+// finish (ticket counter, reset by that block) sums the partials in block order
+// and writes sums[0] = sum of vol * b_P and sums[1] = vol_total (fixed per
+// level).
+constexpr int kRestrictList = 5;   // longest inverse list of one axis (host-checked)
+constexpr int kRestrictStride = 8; // entries reserved per coarse index in the padded lists
+constexpr int kRestrictThreads = 256;
 
+// Padded inverse lists of one axis: fine index and weight e of coarse index I
+// at [I * kRestrictStride + e]; unused entries repeat a valid index with
+// weight 0.
 template <typename T>
-__device__ __forceinline__ double restrict_item(const LevelView<T> &F, const Vec4<T> &rf, const LevelView<T> &Cl,
-                                               const Vec4<T> &bc, const Vec4<T> &xc, const TransferView &tv,
-                                               int scale_p, long t)
+__device__ __forceinline__ void restrict_lists(const AxisMap &m, int I, int idx[kRestrictList], T w[kRestrictList])
 {
-    const int n = Cl.n;
+#pragma unroll
+    for (int e = 0; e < kRestrictList; e++) {
+        idx[e] = __ldg(m.pidx + I * kRestrictStride + e);
+        w[e] = (T)__ldg(m.pw + I * kRestrictStride + e);
+    }
+}
+
+// ws[c * n + v]: sum of the weights of the regular fine rows of coarse row (v, c)
+template <typename T>
+__global__ void k_restrict_weights(LevelView<T> F, LevelView<T> Cl, TransferView tv, T *ws)
+{
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 4L * Cl.n) return;
+    const int c = (int)(t / Cl.n), v = (int)(t % Cl.n);
+    const int J = v % Cl.ny, I = (v / Cl.ny) % Cl.nx, K = v / (Cl.nx * Cl.ny);
+    int xi[kRestrictList], yi[kRestrictList], zi[kRestrictList];
+    T xw[kRestrictList], yw[kRestrictList], zw[kRestrictList];
+    restrict_lists(pick_map(tv.m[0], ax_type(c, 0)), I, xi, xw);
+    restrict_lists(pick_map(tv.m[1], ax_type(c, 1)), J, yi, yw);
+    restrict_lists(pick_map(tv.m[2], ax_type(c, 2)), K, zi, zw);
+    T s = 0;
+    for (int a = 0; a < kRestrictList; a++)
+        for (int d = 0; d < kRestrictList; d++)
+            for (int e = 0; e < kRestrictList; e++) {
+                const int f = zi[a] * (F.nx * F.ny) + xi[d] * F.ny + yi[e];
+                if (!(F.bcm[f] & (1 << c))) s += zw[a] * xw[d] * yw[e];
+            }
+    ws[t] = s;
+}
+
+template <typename T, int kSplit>
+__global__ void __launch_bounds__(kRestrictThreads) k_restrict_compat(
+    LevelView<T> F, Vec4<T> rf, LevelView<T> Cl, Vec4<T> bc, Vec4<T> xc, TransferView tv, int scale_p,
+    const T *__restrict__ wsum, double vol_total, double *partial, unsigned *ticket, double *sums)
+{
+    pdl_enter();
+    constexpr int kPairs = kRestrictThreads / kSplit;
+    __shared__ double sh[32];
+    __shared__ T part[kSplit][kPairs];
+    __shared__ bool last;
+    const int n = Cl.n, pair = threadIdx.x % kPairs, zs = threadIdx.x / kPairs;
+    const long t = (long)blockIdx.x * kPairs + pair;
     double contrib = 0;
+    bool row = false;
+    int c = 0, v = 0, I = 0, J = 0, K = 0;
+    T acc = 0;
     if (t < 4L * n) {
-        const int c = (int)(t / n), v = (int)(t % n);
-        const int J = v % Cl.ny, I = (v / Cl.ny) % Cl.nx, K = v / (Cl.nx * Cl.ny);
-        // component pointers by constant-index selects (no local copy of the parameters)
-        auto comp = [c](const Vec4<T> &V) { return c == 0 ? V.c[0] : (c == 1 ? V.c[1] : (c == 2 ? V.c[2] : V.c[3])); };
-        T *xcc = comp(xc), *bcc = comp(bc);
-        xcc[v] = 0;
-        T out = 0;
-        if (valid_pos(c, I, J, K, Cl.nx, Cl.ny, Cl.nz) && !(Cl.bcm[v] & (1 << c))) {
-            const AxisMap mx = pick_map(tv.m[0], ax_type(c, 0)), my = pick_map(tv.m[1], ax_type(c, 1)),
-                          mz = pick_map(tv.m[2], ax_type(c, 2));
-            T acc = 0, ws = 0;
-            const T etac = c == 0 ? (T)Cl.ec[v] : (T)1;
-            const int x0 = mx.ptr[I], nxq = mx.ptr[I + 1] - x0, y0 = my.ptr[J], nyq = my.ptr[J + 1] - y0;
-            const T *rfc = comp(rf);
-            // the x and y lists (at most kRestrictList entries each, checked on
-            // the host) in registers, the x and y loops unrolled with fixed trip
-            // counts: the fine-node loads of one z line are independent of each
-            // other, so they are issued together rather than one after another
-            int xi[kRestrictList], yi[kRestrictList];
-            T xw[kRestrictList], yw[kRestrictList];
+        c = (int)(t / n);
+        v = (int)(t % n);
+        J = v % Cl.ny;
+        I = (v / Cl.ny) % Cl.nx;
+        K = v / (Cl.nx * Cl.ny);
+        row = valid_pos(c, I, J, K, Cl.nx, Cl.ny, Cl.nz) && !(Cl.bcm[v] & (1 << c));
+    }
+    if (row) {
+        const T *rfc = c == 0 ? rf.c[0] : (c == 1 ? rf.c[1] : (c == 2 ? rf.c[2] : rf.c[3]));
+        const AxisMap mz = pick_map(tv.m[2], ax_type(c, 2));
+        int xi[kRestrictList], yi[kRestrictList];
+        T xw[kRestrictList], yw[kRestrictList];
+        restrict_lists(pick_map(tv.m[0], ax_type(c, 0)), I, xi, xw);
+        restrict_lists(pick_map(tv.m[1], ax_type(c, 1)), J, yi, yw);
 #pragma unroll
-            for (int a = 0; a < kRestrictList; a++) {
-                xi[a] = a < nxq ? mx.idx[x0 + a] : 0;
-                xw[a] = a < nxq ? (T)mx.w[x0 + a] : (T)0;
-                yi[a] = a < nyq ? my.idx[y0 + a] : 0;
-                yw[a] = a < nyq ? (T)my.w[y0 + a] : (T)0;
-            }
-            // the value, mask and viscosity loads of a fine node do not depend
-            // on each other or on a branch: a boundary row contributes with
-            // weight 0 (its value times 0 adds nothing), so every load of a z
-            // line can be in flight at once
-            for (int qz = mz.ptr[K]; qz < mz.ptr[K + 1]; qz++) {
-                const int fk = mz.idx[qz];
-                const T wz = (T)mz.w[qz];
+        for (int q0 = 0; q0 < kRestrictList; q0 += kSplit) {
+            const int q = q0 + zs;
+            if (q >= kRestrictList) break;
+            const T wz = (T)__ldg(mz.pw + K * kRestrictStride + q);
+            const int base = __ldg(mz.pidx + K * kRestrictStride + q) * (F.nx * F.ny);
+            if (wz == (T)0) continue;
+            T line = 0;
 #pragma unroll
-                for (int ax = 0; ax < kRestrictList; ax++) {
-                    if (ax < nxq) {
-                        const T wzx = wz * xw[ax];
-                        const int base = fk * (F.nx * F.ny) + xi[ax] * F.ny;
+            for (int ax = 0; ax < kRestrictList; ax++) {
+                if (xw[ax] == (T)0) continue;
+                const int f = base + xi[ax] * F.ny;
+                T s = 0;
 #pragma unroll
-                        for (int ay = 0; ay < kRestrictList; ay++) {
-                            if (ay < nyq) {
-                                const int f = base + yi[ay];
-                                const bool bnd = __ldg(F.bcm + f) & (1 << c);
-                                T val = __ldg(rfc + f);
-                                if (c == 0 && scale_p) val *= (T)__ldg(F.ec + f);
-                                const T w = bnd ? (T)0 : wzx * yw[ay];
-                                acc += val * w;
-                                ws += w;
-                            }
-                        }
-                    }
+                for (int ay = 0; ay < kRestrictList; ay++) {
+                    if (ay == kRestrictList - 1 && yw[ay] == (T)0) continue;
+                    T val = __ldg(rfc + f + yi[ay]);
+                    if (c == 0 && scale_p) val *= (T)__ldg(F.ec + f + yi[ay]);
+                    s += val * yw[ay];
                 }
+                line += s * xw[ax];
             }
-            // the pressure residuals' viscosity ratio eta_f / eta_c: eta_f per
-            // fine node above, the division by eta_c once here
-            if (c == 0 && scale_p) acc /= etac;
+            acc += line * wz;
+        }
+    }
+    if (kSplit > 1) {
+        if (zs > 0) part[zs][pair] = acc;
+        __syncthreads();
+    }
+    if (zs == 0 && t < 4L * n) {
+#pragma unroll
+        for (int e = 1; e < kSplit; e++) acc += part[e][pair];
+        T out = 0;
+        if (row) {
+            const T ws = wsum[t];
+            // the pressure residuals' viscosity ratio eta_f / eta_c: eta_f per fine node above, the division here
+            if (c == 0 && scale_p) acc /= (T)Cl.ec[v];
             out = ws != (T)0 ? acc / ws : (T)0;
             if (c == 0 && I > 0 && J > 0 && K > 0)
                 contrib = (double)out / ((double)Cl.ax.ih[I] * (double)Cl.ay.ih[J] * (double)Cl.az.ih[K]);
         }
-        bcc[v] = out;
+        (c == 0 ? xc.c[0] : (c == 1 ? xc.c[1] : (c == 2 ? xc.c[2] : xc.c[3])))[v] = 0;
+        (c == 0 ? bc.c[0] : (c == 1 ? bc.c[1] : (c == 2 ? bc.c[2] : bc.c[3])))[v] = out;
     }
-    return contrib;
-}
-template <typename T>
-__global__ void k_restrict_compat(LevelView<T> F, Vec4<T> rf, LevelView<T> Cl, Vec4<T> bc, Vec4<T> xc,
-                                  TransferView tv, int scale_p, double vol_total, double *partial,
-                                  unsigned *ticket, double *sums)
-{
-    pdl_enter();
-    __shared__ double sh[32];
-    __shared__ bool last;
-    const double contrib =
-        restrict_item(F, rf, Cl, bc, xc, tv, scale_p, (long)blockIdx.x * blockDim.x + threadIdx.x);
+    const unsigned pblocks = (unsigned)((n + kPairs - 1) / kPairs);
+    if (blockIdx.x >= pblocks) return;
     const double bsum = block_sum(contrib, sh);
     if (threadIdx.x == 0) {
         partial[blockIdx.x] = bsum;
         __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        last = atomicAdd(ticket, 1u) == pblocks - 1;
     }
     __syncthreads();
     if (last) {
         __threadfence();
         double s = 0;
-        for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) s += ((volatile double *)partial)[q];
+        for (int q = threadIdx.x; q < (int)pblocks; q += blockDim.x) s += ((volatile double *)partial)[q];
         s = block_sum(s, sh);
         if (threadIdx.x == 0) {
             sums[0] = s;
@@ -937,6 +1043,11 @@ __global__ void k_restrict_compat(LevelView<T> F, Vec4<T> rf, LevelView<T> Cl, V
             *ticket = 0;
         }
     }
+}
+inline unsigned restrict_blocks(long n, int split)
+{
+    const long pairs = kRestrictThreads / split;
+    return (unsigned)((4 * n + pairs - 1) / pairs);
 }
 
 // x_f += sum_c w x_c * (p1koef | v1koef) over every fine unknown position.

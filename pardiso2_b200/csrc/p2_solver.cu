@@ -216,6 +216,22 @@ static AxisMap upload_axis(DeviceArena &A, const HostAxis &h, bool restriction =
     m.ptr = upload(A, h.ptr);
     m.idx = upload(A, h.idx);
     m.w = upload(A, h.w);
+    m.pidx = nullptr;
+    m.pw = nullptr;
+    if (restriction) {
+        const size_t nc = h.ptr.size() - 1;
+        std::vector<int> pi(nc * kRestrictStride, 0);
+        std::vector<double> pw(nc * kRestrictStride, 0.0);
+        for (size_t I = 0; I < nc; I++)
+            for (int e = 0; e < kRestrictStride; e++) {
+                const int cnt = h.ptr[I + 1] - h.ptr[I], q = h.ptr[I] + std::min(e, cnt - 1);
+                if (cnt == 0) continue;
+                pi[I * kRestrictStride + e] = h.idx[q];
+                pw[I * kRestrictStride + e] = e < cnt ? h.w[q] : 0.0;
+            }
+        m.pidx = upload(A, pi);
+        m.pw = upload(A, pw);
+    }
     return m;
 }
 
@@ -707,7 +723,7 @@ void Solver::allocate_work()
     {
         long maxc = 1;
         for (int l = 1; l < nl; l++) maxc = std::max<long>(maxc, L[l].n);
-        rpartial = (double *)arena.alloc(sizeof(double) * nblk(4 * maxc));
+        rpartial = (double *)arena.alloc(sizeof(double) * nblk(maxc, kRestrictThreads / 4));
         rticket = (unsigned *)arena.alloc(sizeof(unsigned) * 4);
         for (int l = 0; l < nl; l++) {
             Level &Lv = L[l];
@@ -726,6 +742,20 @@ void Solver::allocate_work()
     scal = (double *)arena.alloc(sizeof(double) * 8);  // [0,1] compat sums, [3] pressure shift
     P2_CUDA_TRY(cudaMallocHost(&hdots_raw, sizeof(double) * HC_LEN));
     hdots.reset(hdots_raw, [](double *p) { cudaFreeHost(p); });
+    // the restriction's weight sums, fixed by the grid and the boundary rows
+    for (int l = 1; l < nl; l++) {
+        Level &F = L[l - 1], &Cl = L[l];
+        const size_t tsz = prm.precision == 0 ? sizeof(float) : sizeof(double);
+        Cl.wsum = arena.alloc(tsz * 4 * (size_t)Cl.n);
+        if (prm.precision == 0) {
+            k_restrict_weights<float><<<nblk(4L * Cl.n), kThreads, 0, st>>>(view<float>(l - 1, false), view<float>(l, false),
+                                                                            F.tv, (float *)Cl.wsum); P2_COUNT_LAUNCH();
+        } else {
+            k_restrict_weights<double><<<nblk(4L * Cl.n), kThreads, 0, st>>>(view<double>(l - 1, false), view<double>(l, false),
+                                                                             F.tv, (double *)Cl.wsum); P2_COUNT_LAUNCH();
+        }
+    }
+    P2_CUDA_TRY(cudaGetLastError());
     // coarse free-unknown set
     build_coarse_index();
 }
@@ -947,7 +977,7 @@ template <typename T>
 void Solver::coarse_approx(Vec4<T> &b, Vec4<T> &x)
 {
     Level &C = L.back();
-    for (int c = 0; c < 4; c++) P2_CUDA_TRY(cudaMemsetAsync(x.c[c], 0, sizeof(T) * C.n, st));
+    P2_CUDA_TRY(cudaMemsetAsync(x.c[0], 0, sizeof(T) * 4 * (size_t)C.n, st));
     const int keep = prm.smoother;
     prm.smoother = 0;
     smooth<T>((int)L.size() - 1, kCoarseApxSweeps);
@@ -1004,31 +1034,24 @@ Vec4<float> &r_of<float>(Level &Lv) { return Lv.r32; }
 template <>
 Vec4<double> &r_of<double>(Level &Lv) { return Lv.r64; }
 
-// FP32 rows run k_rows_zm when its grid has at least this many blocks (8
-// per SM): with fewer, a block's column of planes is a long serial march and
-// the device is not filled (measured at 129^3: 145 against 93 us for k_rows on
-// level 0, 425 blocks; 128 us for 14 MB on level 1, 81 blocks), while at 257^3
-// (2673 blocks) it beats k_rows (0.66 against 0.72 ms).
-constexpr long kZmMinBlocks = 8L * 148;
-
-static long zm_blocks(int nx, int ny, int nz)
-{
-    return (long)((nx + kZmTX - 1) / kZmTX) * ((ny + kZmTY - 1) / kZmTY) * ((nz + kZmKZ - 1) / kZmKZ);
-}
-
+// Operator rows: k_rows, or the z-marching k_rows_zm (variant 2) for
+// cross-checks; k_rows is the faster one on every level (FP32 at 257^3 0.60
+// against 0.64 ms, at 129^3 88 against 150 us; FP64 155 against 242 us).
 template <typename T, typename S>
 static void launch_rows(cudaStream_t st, bool pdl, const LevelView<T> &V, const Fields<T, S> &f, const Vec4<T> &b,
-                        Vec4<T> &out, const Vec4<float> &o32, int mode, int variant = 0)
+                        Vec4<T> &out, const Vec4<float> &o32, const Vec4<S> &copy, int mode, int variant = 0)
 {
-    if (variant == 0) variant = (sizeof(T) == 4 && zm_blocks(V.nx, V.ny, V.nz) >= kZmMinBlocks) ? 2 : 1;
-    if (variant == 1) {
-        if (pdl) pdl_launch(st, nblk(V.n), kThreads, k_rows<T, S>, V, f, b, out, o32, mode);
+    if (variant == 0 || variant == 1) {
+        if (pdl) pdl_launch(st, nblk(V.n, kRowsThreads), kRowsThreads, k_rows<T, S>, V, f, b, out, o32, copy, mode);
         else {
-            k_rows<T, S><<<nblk(V.n), kThreads, 0, st>>>(V, f, b, out, o32, mode);
+            k_rows<T, S><<<nblk(V.n, kRowsThreads), kRowsThreads, 0, st>>>(V, f, b, out, o32, copy, mode);
             P2_COUNT_LAUNCH();
         }
         return;
     }
+    for (int c = 0; copy.c[0] && c < 4; c++)
+        P2_CUDA_TRY(cudaMemcpyAsync(copy.c[c], c == 0 ? f.p : c == 1 ? f.vx : c == 2 ? f.vy : f.vz, sizeof(S) * (size_t)V.n,
+                                    cudaMemcpyDeviceToDevice, st));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1247,10 +1270,25 @@ void Solver::level_residual(int l)
     Vec4<T> &x = vx_of<T>(Lv, 0), &b = b_of<T>(Lv), &r = r_of<T>(Lv);
     Fields<T, T> f{x.c[0], x.c[1], x.c[2], x.c[3]};
     Vec4<float> none;
-    launch_rows<T, T>(st, true, V, f, b, r, none, 0, dbg_rows_variant);
-    if (Lv.nbc)
-        pdl_launch(st, nblk(Lv.nbc), kThreads, k_bc_rows<T, T>, Lv.nbc, (const int *)Lv.bu, (const int *)Lv.bt,
-                   (const float *)Lv.bk, f, b, r, none, 0);
+    // the restriction takes no residual from boundary rows: they stay 0
+    launch_rows<T, T>(st, true, V, f, b, r, none, Vec4<T>(), 0, dbg_rows_variant);
+}
+
+// Restriction of level l to l + 1: the z lists of a coarse unknown split over
+// four threads where one thread each would not fill the device (one block of
+// 1024 an SM); beyond that the split only repeats the list reads (257^3: 1.43
+// against 0.63 ms).
+constexpr long kRestrictSplitMax = 148L * 1024;  // coarse unknowns
+template <typename T>
+void Solver::launch_restrict(int l, const Vec4<T> &r, const Vec4<T> &b, const Vec4<T> &x, const T *ws)
+{
+    Level &F = L[l], &Cl = L[l + 1];
+    auto go = [&](auto kern, int split) {
+        pdl_launch(st, restrict_blocks(Cl.n, split), kRestrictThreads, kern, view<T>(l, false), r, view<T>(l + 1, false), b, x,
+                   F.tv, 1, ws, Cl.compat_vol, rpartial, rticket, scal);
+    };
+    if (4L * Cl.n <= kRestrictSplitMax) go(k_restrict_compat<T, 4>, 4);
+    else go(k_restrict_compat<T, 1>, 1);
 }
 
 template <typename T>
@@ -1261,9 +1299,8 @@ void Solver::vcycle()
         smooth<T>(l, prm.npre[l]);
         level_residual<T>(l);
         Level &F = L[l], &Cl = L[l + 1];
-        LevelView<T> VF = view<T>(l, false), VC = view<T>(l + 1, false);
-        pdl_launch(st, nblk(4L * Cl.n), kThreads, k_restrict_compat<T>, VF, r_of<T>(F), VC, b_of<T>(Cl),
-                   vx_of<T>(Cl, 0), F.tv, 1, Cl.compat_vol, rpartial, rticket, scal);
+        LevelView<T> VC = view<T>(l + 1, false);
+        launch_restrict<T>(l, r_of<T>(F), b_of<T>(Cl), vx_of<T>(Cl, 0), (const T *)Cl.wsum);
         pdl_launch(st, nblk(Cl.n), kThreads, k_compat_apply<T>, VC, b_of<T>(Cl).c[0], (const double *)scal);
     }
     if (nl > 1) coarse_solve<T>(b_of<T>(L[nl - 1]), vx_of<T>(L[nl - 1], 0));
@@ -1325,15 +1362,15 @@ double Solver::residual_norm2()
 }
 
 // out = b - A x (mode 0) or A x (mode 1) on level 0 in FP64 (x stored as
-// S); r32 optional.
+// S); a float copy of out and a copy of x optional.
 template <typename S>
-void Solver::rows0(const Vec4<S> &x, Vec4<double> &out, Vec4<float> *r32, int mode)
+void Solver::rows0(const Vec4<S> &x, Vec4<double> &out, Vec4<float> *r32, int mode, const Vec4<S> *copy)
 {
     Level &L0 = L[0];
     LevelView<double> V = view<double>(0, true);
     Fields<double, S> f{x.c[0], x.c[1], x.c[2], x.c[3]};
     Vec4<float> o32 = r32 ? *r32 : Vec4<float>();
-    launch_rows<double, S>(st, false, V, f, gb, out, o32, mode, dbg_rows_variant);
+    launch_rows<double, S>(st, false, V, f, gb, out, o32, copy ? *copy : Vec4<S>(), mode, dbg_rows_variant);
     if (L0.nbc) {
         k_bc_rows<double, S><<<nblk(L0.nbc), kThreads, 0, st>>>(L0.nbc, L0.bu, L0.bt, L0.bk, f, gb, out, o32, mode);
         P2_COUNT_LAUNCH();
@@ -1347,10 +1384,10 @@ void Solver::precondition()
 {
     Level &L0 = L[0];
     if (prm.precision == 0) {
-        for (int c = 0; c < 4; c++) P2_CUDA_TRY(cudaMemsetAsync(L0.x32.c[c], 0, sizeof(float) * L0.n, st));
+        P2_CUDA_TRY(cudaMemsetAsync(L0.x32.c[0], 0, sizeof(float) * 4 * (size_t)L0.n, st));
         run_vcycle_graph<float>();
     } else {
-        for (int c = 0; c < 4; c++) P2_CUDA_TRY(cudaMemsetAsync(L0.x64.c[c], 0, sizeof(double) * L0.n, st));
+        P2_CUDA_TRY(cudaMemsetAsync(L0.x64.c[0], 0, sizeof(double) * 4 * (size_t)L0.n, st));
         run_vcycle_graph<double>();
     }
 }
@@ -1457,11 +1494,9 @@ p2_solve_info Solver::solve()
             // Z_k = the correction, W_{k+1} = A Z_k, orthogonalised
             Vec4<double> &q = W[k + 1];
             if (f32) {
-                P2_CUDA_TRY(cudaMemcpyAsync(Z32[k].c[0], L0.x32.c[0], vec64 / 2, cudaMemcpyDeviceToDevice, st));
-                rows0(L0.x32, q, nullptr, 1);
+                rows0(L0.x32, q, nullptr, 1, &Z32[k]);
             } else {
-                P2_CUDA_TRY(cudaMemcpyAsync(Z64[k].c[0], L0.x64.c[0], vec64, cudaMemcpyDeviceToDevice, st));
-                rows0(L0.x64, q, nullptr, 1);
+                rows0(L0.x64, q, nullptr, 1, &Z64[k]);
             }
             P2_CUDA_TRY(launch_basis_dots(st, k + 1, n2, q.c[0], B, L0.pin, partial, dticket, ww, hcol)); P2_COUNT_LAUNCH();
             if (f32)
@@ -1795,7 +1830,7 @@ void Solver::debug_apply(int l, const double *x, double *y)
     LevelView<double> V = view<double>(l, l == 0);
     Fields<double, double> f{X.v.c[0], X.v.c[1], X.v.c[2], X.v.c[3]};
     Vec4<float> none;
-    launch_rows<double, double>(st, false, V, f, B.v, Y.v, none, 1, dbg_rows_variant);
+    launch_rows<double, double>(st, false, V, f, B.v, Y.v, none, Vec4<double>(), 1, dbg_rows_variant);
     if (Lv.nbc)
         k_bc_rows<double, double><<<nblk(Lv.nbc), kThreads, 0, st>>>(Lv.nbc, Lv.bu, Lv.bt, Lv.bk, f, B.v, Y.v, none, 1); P2_COUNT_LAUNCH();
     P2_CUDA_TRY(cudaGetLastError());
@@ -1816,11 +1851,20 @@ void Solver::debug_restrict(int lc, const double *fine_res, double *coarse_rhs, 
     debug_prepare();
     Level &F = L[lc - 1], &Cl = L[lc];
     TmpVec R(F.n), Bc(Cl.n), Xc(Cl.n);
-    to_vec4(st, fine_res, F.n, R.v);
     LevelView<double> VF = view<double>(lc - 1, false), VC = view<double>(lc, false);
-    // the V-cycle's restriction kernel (with its fused compatibility sums)
-    k_restrict_compat<double><<<nblk(4L * Cl.n), kThreads, 0, st>>>(VF, R.v, VC, Bc.v, Xc.v, F.tv, 1, Cl.compat_vol,
-                                                                     rpartial, rticket, scal); P2_COUNT_LAUNCH();
+    // the V-cycle's restriction kernel (with its fused compatibility sums), whose residuals are 0 on boundary rows
+    {
+        std::vector<double> r(fine_res, fine_res + 4 * (size_t)F.n);
+        for (int u = 0; u < F.n; u++)
+            for (int c = 0; c < 4; c++)
+                if (F.h_bcm[u] & (1 << c)) r[4 * (size_t)u + c] = 0.0;
+        to_vec4(st, r.data(), F.n, R.v);
+    }
+    double *ws = nullptr;
+    P2_CUDA_TRY(cudaMalloc(&ws, sizeof(double) * 4 * (size_t)Cl.n));
+    struct Free { void *p; ~Free() { cudaFree(p); } } hold{ws};
+    k_restrict_weights<double><<<nblk(4L * Cl.n), kThreads, 0, st>>>(VF, VC, F.tv, ws); P2_COUNT_LAUNCH();
+    launch_restrict<double>(lc - 1, R.v, Bc.v, Xc.v, ws);
     if (compat) {
         k_compat_apply<double><<<nblk(Cl.n), kThreads, 0, st>>>(VC, Bc.v.c[0], scal); P2_COUNT_LAUNCH();
     }
@@ -1971,14 +2015,8 @@ double Solver::debug_time_stage(int stage, int l, int variant, int reps)
                 else rows0(Z64[0], W[1], nullptr, 1);
             } else if (stage == 2) {
                 Level &F = L[l], &Cl = L[l + 1];
-                if (f32)
-                    pdl_launch(st, nblk(4L * Cl.n), kThreads, k_restrict_compat<float>, view<float>(l, false), F.r32,
-                               view<float>(l + 1, false), Cl.b32, Cl.x32, F.tv, 1, Cl.compat_vol, rpartial, rticket,
-                               scal);
-                else
-                    pdl_launch(st, nblk(4L * Cl.n), kThreads, k_restrict_compat<double>, view<double>(l, false),
-                               F.r64, view<double>(l + 1, false), Cl.b64, Cl.x64, F.tv, 1, Cl.compat_vol, rpartial,
-                               rticket, scal);
+                if (f32) launch_restrict<float>(l, F.r32, Cl.b32, Cl.x32, (const float *)Cl.wsum);
+                else launch_restrict<double>(l, F.r64, Cl.b64, Cl.x64, (const double *)Cl.wsum);
             } else {
                 Level &F = L[l], &Cl = L[l + 1];
                 if (f32)

@@ -40,6 +40,7 @@ struct Level {
     std::vector<uint8_t> h_bcm;
     int pin = -1;
     double pinval = 0;
+    void *wsum = nullptr;         // restriction weight sums of this (coarse) level's rows, the V-cycle's type
     double compat_vol = 0;        // total volume of the non-boundary pressure cells
     // stored cell factors of the full cell-block smoother: per colour
     // kBlkEntries x blk_stride values of the V-cycle's type, entry-major
@@ -225,6 +226,8 @@ class Solver {
     void factor_cells();
     template <typename T>
     void level_residual(int l);
+    template <typename T>
+    void launch_restrict(int l, const Vec4<T> &r, const Vec4<T> &b, const Vec4<T> &x, const T *ws);
 
     template <typename T>
     void vcycle();
@@ -234,7 +237,7 @@ class Solver {
     void capture_vcycle_graph();
     void set_nodes_device();
     template <typename S>
-    void rows0(const Vec4<S> &x, Vec4<double> &out, Vec4<float> *r32, int mode);
+    void rows0(const Vec4<S> &x, Vec4<double> &out, Vec4<float> *r32, int mode, const Vec4<S> *copy = nullptr);
     void precondition();
     std::vector<cudaEvent_t> vc_ev;  // V-cycle timing events of a solve (reused)
     double residual_norm2();
