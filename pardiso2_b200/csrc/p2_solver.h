@@ -247,6 +247,7 @@ class Solver {
     void debug_prepare();
     Grid3 grid3() const;
     void ensure_move_buffers(long nmark);
+    void reserve_move_positions(long nmark);
     void velocity_f32();
 
     void heat_smooth(int l, int sweeps, double t0koef);
