@@ -364,4 +364,9 @@ struct TransferView {
     AxisMap m[3][3];  // [axis][type]
 };
 
+struct BcFollow {
+    int n;
+    const int *uc, *target;
+    const float *k;
+};
 }  // namespace p2

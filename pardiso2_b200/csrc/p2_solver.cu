@@ -40,14 +40,15 @@ constexpr int kCoarseApxSweeps = 16;
 // cell planes per block of the fused sweep (each block starts 3 planes early)
 constexpr int kSweepChunk = 32;
 // Outer iterations that use the smoothed coarsest level: kOverlapScale *
-// nF / n0, the inverse's time over the fine work of one iteration (linear in
-// n0), fixed from the grid sizes so that the iterates do not depend on timing
-// (5 at 65^3, where the inverse takes 4.3 ms, 1 at 129^3, 0 at 257^3, all with
-// nF = 3644); none on grids of fewer than four levels, where the
-// coarsest level is too large a part of the problem for smoothing to stand
-// in for it.  The solve waits for the LU at that iteration if it is still
-// running.
-constexpr double kOverlapScale = 400.0;
+// nF / n0, fixed from the grid sizes so that the iterates do not depend on
+// timing (6 at 33^3, 0 from 65^3 on, all with nF = 3644).  The inverse
+// fills the device, so running it beside the V-cycles gains little, and each
+// such iteration reduces the residual less: 33^3 8.3 ms without, 8.0 ms with 6, 9.0
+// ms with 16; 65^3 41.4 / 49.1 ms (two models) without, 45.9 / 52.5 ms with 5.
+// None on grids of one or two levels, where the coarsest level is too large a
+// part of the problem for smoothing to stand in for it.  The solve waits for the
+// inverse at that iteration if it is still running.
+constexpr double kOverlapScale = 60.0;
 constexpr int kOverlapMax = 16;
 void d2f(cudaStream_t st, size_t n, const double *a, float *b);
 size_t gj_work_doubles(int n);
@@ -594,6 +595,20 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
             Lv.sw_order = upload(arena, order);
         }
         build_resident(Lv);
+        if (!Lv.res_mode) {
+            std::vector<int> slot(Lv.h_bu.size(), -1), uc, target;
+            std::vector<float> k;
+            for (size_t q = 0; q < Lv.h_bu.size(); q++) {
+                if (Lv.h_rt[q] < 0) continue;
+                slot[q] = (int)uc.size();
+                uc.push_back(Lv.h_bu[q]);
+                target.push_back(Lv.h_rt[q]);
+                k.push_back((float)Lv.h_rk[q]);
+            }
+            Lv.follow = BcFollow{(int)uc.size(), upload(arena, uc), upload(arena, target), upload(arena, k)};
+            Lv.follow_slot = upload(arena, slot);
+            Lv.follow_const = arena.alloc(sizeof(double) * std::max<size_t>(uc.size(), 1));
+        }
         Lv.h_bcm = m;
         Lv.bcm = upload(arena, m);
         Lv.bu = upload(arena, bu);
@@ -959,8 +974,8 @@ void Solver::coarse_setup()
     gj_inverse(st_lu, A_c, gj, Ainv64, prm.precision == 0 ? Ainv32 : nullptr, gj_work, d_info, &lu_graph);
     P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
     lu_pending = true;
-    lu_overlap_iters = L.size() < 4 ? 0
-                       : (int)std::min<double>(kOverlapMax, std::floor(kOverlapScale * nF / (double)L[0].n + 0.5));
+    lu_overlap_iters = L.size() < 3 ? 0
+                       : (int)std::min<double>(kOverlapMax, kOverlapScale * nF / (double)L[0].n);
 }
 
 // The inverse by the pivoted band LU (A_c is overwritten), brought into the
@@ -1251,7 +1266,7 @@ void Solver::smooth(int l, int sweeps)
         else smooth_resident<T, false>(l, sweeps);
         return;
     }
-    bc_set<T>(l, x, b);
+    if (sweeps <= 0 || use_fused(l) || Lv.res_mode) bc_set<T>(l, x, b);
     if (sweeps <= 0) return;
     // colour 0 reads velocities from x and writes y, colour 1 goes back; the
     // pressure is updated in place in x.c[0] (yy shares it)
@@ -1277,11 +1292,18 @@ void Solver::smooth(int l, int sweeps)
         }
         return;
     }
+    const bool follow = !Lv.res_mode && Lv.nbc > 0;
+    if (follow)
+        pdl_launch(st, nblk(Lv.nbc), kThreads, k_bc_begin<T>, Lv.nbc, (const int *)Lv.bu, (const int *)Lv.bt,
+                   (const float *)Lv.bk, (const int *)Lv.bnext, (const int *)Lv.follow_slot, x, yy, b,
+                   (T *)Lv.follow_const);
     for (int s = 0; s < sweeps; s++) {
         for (int col = 0; col < 2; col++) {
             Vec4<T> &vin = col ? yy : x, &vout = col ? x : yy;
             smoother_pass<T>(l, V, x.c[0], vin, vout, b, col);
-            bc_set<T>(l, vout, b);
+            if (!follow) bc_set<T>(l, vout, b);
+            else if (Lv.follow.n > 0)
+                pdl_launch(st, nblk(Lv.follow.n), kThreads, k_bc_follow<T>, Lv.follow, (const T *)Lv.follow_const, vout);
         }
     }
 }

@@ -56,6 +56,10 @@ struct Level {
     int res_mode = 0, res_blocks = 0, res_slots = 0, res_cap = 0;
     int *res_ptr = nullptr;
     int4 *res_dep = nullptr;
+    // boundary rows between separate colour passes
+    BcFollow follow{};
+    int *follow_slot = nullptr;
+    void *follow_const = nullptr;
     // boundary rows sorted by copy-chain depth
     int nbc = 0;
     std::vector<int> bc_groups;
