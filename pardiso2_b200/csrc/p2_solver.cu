@@ -86,52 +86,28 @@ static void pdl_launch(cudaStream_t st, dim3 grid, dim3 block, void (*kern)(KArg
     pdl_launch_smem(st, grid, block, 0, kern, std::forward<Args>(args)...);
 }
 
-static void *zeroed_malloc(size_t bytes)
+void *DeviceArena::alloc(size_t bytes)
 {
     void *p = nullptr;
+    if (bytes == 0) bytes = 16;
+    bytes += guard;
     cudaError_t e = cudaMalloc(&p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         throw Error(P2_ERR_NOMEM, "cudaMalloc of " + std::to_string(bytes) + " bytes failed");
     }
+    ptrs.push_back(p);
     // Zero-fill on the legacy stream and wait for it: the library's own
     // streams are non-blocking, so without the wait a fill still in flight
     // could land after a copy that the caller queues on its stream.
-    e = cudaMemsetAsync(p, 0, bytes, 0);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-    if (e != cudaSuccess) {
-        cudaFree(p);
-        P2_CUDA_TRY(e);
-    }
-    return p;
-}
-// Small requests (tables, coarse levels) share blocks of kArenaChunk bytes,
-// so that a grid's set-up costs tens of allocations instead of hundreds.
-constexpr size_t kArenaChunk = (size_t)8 << 20, kArenaSmall = (size_t)1 << 20;
-void *DeviceArena::alloc(size_t bytes)
-{
-    const size_t need = (std::max<size_t>(bytes, 16) + guard + 255) / 256 * 256;
-    if (need > kArenaSmall) {
-        void *p = zeroed_malloc(need);
-        ptrs.push_back(p);
-        return p;
-    }
-    if (left < need) {
-        chunk = (char *)zeroed_malloc(kArenaChunk);
-        ptrs.push_back(chunk);
-        left = kArenaChunk;
-    }
-    void *p = chunk;
-    chunk += need;
-    left -= need;
+    P2_CUDA_TRY(cudaMemsetAsync(p, 0, bytes, 0));
+    P2_CUDA_TRY(cudaStreamSynchronize(0));
     return p;
 }
 void DeviceArena::release()
 {
     for (void *p : ptrs) cudaFree(p);
     ptrs.clear();
-    chunk = nullptr;
-    left = 0;
 }
 
 // ---------------------------------------------------------------------------

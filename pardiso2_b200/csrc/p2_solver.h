@@ -14,8 +14,6 @@ namespace p2 {
 struct DeviceArena {
     std::vector<void *> ptrs;
     size_t guard = 0;  // zero-filled bytes appended to every allocation
-    char *chunk = nullptr;  // rest of the block that small allocations share
-    size_t left = 0;
     void *alloc(size_t bytes);
     void release();
 };
