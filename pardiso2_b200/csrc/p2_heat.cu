@@ -35,12 +35,14 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <thread>
 #include <vector>
 
 #include "p2_internal.cuh"
 #include "p2_interp.cuh"
 #include "p2_solver.h"
+#include "p2_stage.h"
 
 namespace p2 {
 
@@ -734,6 +736,8 @@ void Solver::heat_set_bc(const int *bondm, long bondm_len, const float *bondv1, 
         heat.mev_owner.reset(e2, [](CUevent_st *p) { cudaEventDestroy(p); });
         heat.mev = e2;
     }
+    heat.stage = std::make_shared<HostStage>();
+    heat.stage->reserve();
     P2_CUDA_TRY(cudaMallocHost((void **)&heat.host, sizeof(double) * 8));  // [0..3] error, range; [4] sub-step
     heat.host_owner.reset(heat.host, [](double *p) { cudaFreeHost(p); });
     P2_CUDA_TRY(cudaStreamSynchronize(st));
@@ -820,19 +824,19 @@ p2_heat_info Solver::titerate(const p2_heat_params &hp, double timestep, float *
     info.tktimestep = 1e30;
     heat.kernels = 0;
     P2_CUDA_TRY(cudaEventRecord(ev[0], st));
-    P2_CUDA_TRY(cudaMemcpyAsync(heat.tk, tk, fb, cudaMemcpyHostToDevice, st));
-    P2_CUDA_TRY(cudaMemcpyAsync(heat.kt, kt, fb, cudaMemcpyHostToDevice, st));
-    P2_CUDA_TRY(cudaMemcpyAsync(heat.cp, cp, fb, cudaMemcpyHostToDevice, st));
-    P2_CUDA_TRY(cudaMemcpyAsync(heat.ro, ro, fb, cudaMemcpyHostToDevice, st));
-    P2_CUDA_TRY(cudaMemcpyAsync(heat.ht, ht, fb, cudaMemcpyHostToDevice, st));
-    P2_CUDA_TRY(cudaMemcpyAsync(heat.et, et, fb, cudaMemcpyHostToDevice, st));
-    if (hp.adiabyn) {
-        const float *v[3] = {vx, vy, vz};
-        for (int a = 0; a < 3; a++) P2_CUDA_TRY(cudaMemcpyAsync(heat.vel[a], v[a], fb, cudaMemcpyHostToDevice, st));
+    {
+        auto host = [](const void *p) { return const_cast<void *>(p); };
+        std::vector<HostCopy> in = {{heat.tk, host(tk), fb}, {heat.kt, host(kt), fb}, {heat.cp, host(cp), fb},
+                                    {heat.ro, host(ro), fb}, {heat.ht, host(ht), fb}, {heat.et, host(et), fb}};
+        if (hp.adiabyn) {
+            const float *v[3] = {vx, vy, vz};
+            for (int a = 0; a < 3; a++) in.push_back({heat.vel[a], host(v[a]), fb});
+        }
+        if (hp.adiabyn == 2) in.push_back({heat.pr, host(pr), sizeof(double) * n0});
+        if (hp.frictyn)
+            for (int q = 0; q < 12; q++) in.push_back({heat.se[q], host(se[q]), fb});
+        P2_CUDA_TRY(heat.stage->run(dev, std::move(in), cudaMemcpyHostToDevice, st));
     }
-    if (hp.adiabyn == 2) P2_CUDA_TRY(cudaMemcpyAsync(heat.pr, pr, sizeof(double) * n0, cudaMemcpyHostToDevice, st));
-    if (hp.frictyn)
-        for (int q = 0; q < 12; q++) P2_CUDA_TRY(cudaMemcpyAsync(heat.se[q], se[q], fb, cudaMemcpyHostToDevice, st));
 
     GridSh G;
     for (int a = 0; a < 3; a++) {
@@ -875,8 +879,7 @@ p2_heat_info Solver::titerate(const p2_heat_params &hp, double timestep, float *
         return info;
     }
     // The markers are needed only after the last sub-step: a helper thread
-    // copies them on a second stream while the sub-steps run (the copies
-    // from pageable memory block the thread that issues them).
+    // copies them on a second stream while the sub-steps run.
     struct Uploader {
         std::thread th;
         cudaError_t err = cudaSuccess;
@@ -902,12 +905,16 @@ p2_heat_info Solver::titerate(const p2_heat_params &hp, double timestep, float *
         const HeatState *H = &heat;
         up.th = std::thread([u, H, device, nmark, mx, my, mz, mt, markk] {
             const size_t mb = sizeof(float) * nmark;
+            auto host = [](const void *p) { return const_cast<void *>(p); };
             cudaError_t e = cudaSetDevice(device);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(H->mx, mx, mb, cudaMemcpyHostToDevice, H->mst);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(H->my, my, mb, cudaMemcpyHostToDevice, H->mst);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(H->mz, mz, mb, cudaMemcpyHostToDevice, H->mst);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(H->mk, markk, mb, cudaMemcpyHostToDevice, H->mst);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(H->mt, mt, nmark, cudaMemcpyHostToDevice, H->mst);
+            try {
+                if (e == cudaSuccess)
+                    e = H->stage->run(device, {{H->mx, host(mx), mb}, {H->my, host(my), mb}, {H->mz, host(mz), mb},
+                                               {H->mk, markk, mb}, {H->mt, host(mt), (size_t)nmark}},
+                                      cudaMemcpyHostToDevice, H->mst);
+            } catch (...) {
+                e = cudaErrorMemoryAllocation;
+            }
             if (e == cudaSuccess) e = cudaEventRecord(H->mev, H->mst);
             u->err = e;
         });
@@ -998,10 +1005,10 @@ p2_heat_info Solver::titerate(const p2_heat_params &hp, double timestep, float *
             k_heat_anti<<<hb(nmark), 256, 0, st>>>(M);
             heat.kernels += 2;
         }
-        P2_CUDA_TRY(cudaMemcpyAsync(markk, heat.mk, mb, cudaMemcpyDeviceToHost, st));
+        P2_CUDA_TRY(heat.stage->run(dev, {{heat.mk, markk, mb}}, cudaMemcpyDeviceToHost, st));
         P2_CUDA_TRY(cudaMemcpyAsync(heat.host + 6, heat.scal + 6, sizeof(double), cudaMemcpyDeviceToHost, st));
     }
-    P2_CUDA_TRY(cudaMemcpyAsync(tk, heat.tk, fb, cudaMemcpyDeviceToHost, st));
+    P2_CUDA_TRY(heat.stage->run(dev, {{heat.tk, tk, fb}}, cudaMemcpyDeviceToHost, st));
     P2_CUDA_TRY(cudaEventRecord(ev[1], st));
     P2_CUDA_TRY(cudaEventSynchronize(ev[1]));
     P2_CUDA_TRY(cudaGetLastError());

@@ -93,6 +93,7 @@ struct HeatLevel {
     AxisMap map[3]{};                     // this level -> next coarser level
 };
 
+class HostStage;
 struct HeatState {
     bool ready = false;
     std::vector<HeatLevel> lv;
@@ -105,6 +106,7 @@ struct HeatState {
     double *partial = nullptr, *scal = nullptr, *S0 = nullptr, *S1 = nullptr;
     double *host = nullptr;
     std::shared_ptr<double> host_owner;
+    std::shared_ptr<HostStage> stage;  // pageable arrays of a call
     long mcap = 0;
     float *mx = nullptr, *my = nullptr, *mz = nullptr, *mk = nullptr;
     signed char *mt = nullptr;
