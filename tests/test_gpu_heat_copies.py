@@ -19,7 +19,7 @@ def test_pageable_and_page_locked_arrays():
     m = heat_model()
     th, vel, se, pr, _, _ = heat_inputs(m)
     v = HEAT_VARIANTS["mg"]
-    d = dict(HEAT_COMMON, **v, max_cycles=200, heatdif=0.0)
+    d = {**HEAT_COMMON, **v, "max_cycles": 200, "heatdif": 0.0}
     hp = capi.heat_params(**{k: d[k] for k in ("maxtkstep", "heatmin", "t0koef", "t1koef", "heatdif", "tdeep", "zdeep",
                                                "multinumt", "multicyct", "frictyn", "adiabyn", "max_cycles", "pre", "post")})
     n = 13 * PIECE + 7
