@@ -14,6 +14,7 @@
 //   residual                         k_heat_resid    gausmatt 1103-1119
 //   residual restriction             k_heat_restrict trestrict 1122-1233
 //   correction prolongation          k_heat_prolong  tprolong 954-1054
+//   the two above, level resident    k_heat_sweeps
 //   error and float temperatures     k_heat_error    heaterr mode 2 (250-289),
 //                                                    the reload 505-512
 //   marker temperatures              k_heat_markers  641-768 with tkcalc1
@@ -39,6 +40,7 @@
 #include <thread>
 #include <vector>
 
+#include "p2_barrier.cuh"
 #include "p2_internal.cuh"
 #include "p2_interp.cuh"
 #include "p2_solver.h"
@@ -303,10 +305,105 @@ __global__ void __launch_bounds__(256) k_heat_resid(HeatLv L, HeatBc B, int leve
     L.r[u] = t >= 0 ? (c - L.x[u]) + B.bk[q - 1] * L.x[t] : c - L.x[u];
 }
 
+// All sweeps of a smoothing call in one launch, with the residual after them
+// where the next kernel restricts it: the operations of k_heat_gs and
+// k_heat_resid in the same order, so the iterates are the same to the last bit.
+// A pass on a level of up to about 65^3 nodes is latency: as a launch of its own
+// it waits for the launch, for the coefficients from L2 and for a chain of
+// sums and a division.  Here a thread keeps the coefficients, the right-hand
+// side and the unknown of one node of each colour in registers for the whole
+// call, and one boundary row; a pass loads the six neighbours and ends in a
+// barrier.  A pass as a launch / resident: one block 2.9 / 0.9 us (11^3 nodes),
+// a cluster 2.7 / 2.1 (13^3), 2.9 / 2.5 (31 x 33 x 31), the grid 3.0 / 2.8
+// (37^3), 3.7 / 3.3 (65^3); the step on 65^3 nodes 5.6 -> 4.5 ms between its
+// events without markers, 982 -> 232 launches.
+enum { kHeatBlock = 0, kHeatCluster = 1, kHeatGrid = 2 };
+constexpr int kHeatThreads = 1024;  // of a block at most: 64 registers each
+constexpr int kHeatClusterSize = 16;
+
+template <int kForm>
+__global__ void __launch_bounds__(kHeatThreads, 1) k_heat_sweeps(HeatLv L, HeatBc B, int sweeps, double t0koef,
+                                                                 int level0, int resid, GridBarrier S)
+{
+    __shared__ bool ok;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nyh = (L.ny + 1) / 2, ny = L.ny, nxy = L.nx * L.ny, nh = (int)L.nh;
+    double a[2][7], b[2], x[2];
+    int u[2];
+    // other blocks' nodes: past the L1, which is not coherent with theirs
+    auto ld = [](const double *p) { return kForm == kHeatBlock ? *p : __ldcg(p); };
+    {
+        const int jj = t % nyh, rest = t / nyh, i = rest % L.nx, k = rest / L.nx;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const int j = 2 * jj + ((i + k + c) & 1);
+            const double *p = L.a + (c * nh + t);
+            a[c][0] = t < nh && j < ny ? *p : 0.0;
+            u[c] = k * nxy + i * ny + j;
+            if (a[c][0] == 0) continue;  // boundary row
+#pragma unroll
+            for (int q = 1; q < 7; q++) a[c][q] = p[(long)q * 2 * nh];
+            b[c] = L.b[c * nh + t];
+            x[c] = L.x[u[c]];
+        }
+    }
+    int bu = 0, bt = 0, bpass = -1;
+    double bk = 0, bc = 0;
+    if (t < B.nbc) {
+        bu = B.bu[t]; bt = B.bt[t]; bk = B.bk[t]; bpass = B.bpass[t];
+        bc = level0 ? B.bconst[t] : 0.0;
+    }
+    auto ax = [&](int c, double s) {
+        const double *p = L.x + u[c];
+        const double x1 = ld(p - ny), x2 = ld(p + ny), x3 = ld(p - 1), x4 = ld(p + 1), x5 = ld(p - nxy), x6 = ld(p + nxy);
+        s += a[c][0] * x[c];
+        s += a[c][1] * x1;
+        s += a[c][2] * x2;
+        s += a[c][3] * x3;
+        s += a[c][4] * x4;
+        s += a[c][5] * x5;
+        s += a[c][6] * x6;
+        return s;
+    };
+    unsigned target = 0;
+    auto sync = [&] {
+        if (kForm == kHeatBlock) {
+            __syncthreads();
+            return true;
+        }
+        return res_sync<kForm == kHeatCluster>(S, target, &ok);
+    };
+    bool go = true;
+    for (int s = 0; go && s < sweeps; s++) {
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            if (bpass == c) L.x[bu] = bt >= 0 ? bc + bk * ld(L.x + bt) : bc;
+            if (a[c][0] != 0) {
+                const double ival = ax(c, -b[c]);
+                x[c] -= ival / a[c][0] * t0koef;
+                L.x[u[c]] = x[c];
+            }
+            if (go && (c == 0 || s + 1 < sweeps || resid)) go = sync();
+        }
+    }
+    if (go && resid) {
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+            if (a[c][0] != 0) L.r[u[c]] = b[c] - (ax(c, 0.0));
+        if (bpass >= 0) {
+            const double xu = ld(L.x + bu);
+            L.r[bu] = bt >= 0 ? (bc - xu) + bk * ld(L.x + bt) : bc - xu;
+        }
+    }
+    if (kForm == kHeatGrid) res_leave(S);
+}
+
 // trestrict: coarse right-hand side = weighted mean of the fine residuals
 // over the heat rows of the coarse level, 0 on its boundary rows; coarse
-// solution reset to 0.
-__global__ void k_heat_restrict(HeatLv F, HeatLv C, AxisMap mx, AxisMap my, AxisMap mz)
+// solution reset to 0.  The lists hold at most kHeatList nodes per axis where the
+// lines coarsen as the configurations' do.
+constexpr int kHeatList = 4;
+__global__ void __launch_bounds__(128) k_heat_restrict(HeatLv F, HeatLv C, AxisMap mx, AxisMap my, AxisMap mz)
 {
     const long u = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= C.n) return;
@@ -316,16 +413,48 @@ __global__ void k_heat_restrict(HeatLv F, HeatLv C, AxisMap mx, AxisMap my, Axis
     const long ci = heat_ci(C, c1, c2, c3);
     if (C.bci[u]) { C.b[ci] = 0; return; }
     double num = 0, den = 0;
-    for (int qz = mz.ptr[c3]; qz < mz.ptr[c3 + 1]; qz++) {
-        const double wz = mz.w[qz];
-        const long oz = (long)mz.idx[qz] * fnxy;
-        for (int qx = mx.ptr[c1]; qx < mx.ptr[c1 + 1]; qx++) {
-            const double wx = mx.w[qx];
-            const long ox = oz + (long)mx.idx[qx] * F.ny;
-            for (int qy = my.ptr[c2]; qy < my.ptr[c2 + 1]; qy++) {
-                const double swt = wx * my.w[qy] * wz;
-                num += F.r[ox + my.idx[qy]] * swt;
-                den += swt;
+    const int x0 = mx.ptr[c1], nx = mx.ptr[c1 + 1] - x0, y0 = my.ptr[c2], ny = my.ptr[c2 + 1] - y0;
+    if (nx <= kHeatList && ny <= kHeatList) {
+        // a plane's residuals all in flight, added in the lists' order
+        int ix[kHeatList], iy[kHeatList];
+        double wx[kHeatList], wy[kHeatList];
+#pragma unroll
+        for (int e = 0; e < kHeatList; e++) {
+            ix[e] = e < nx ? mx.idx[x0 + e] : 0;
+            wx[e] = e < nx ? mx.w[x0 + e] : 0;
+            iy[e] = e < ny ? my.idx[y0 + e] : 0;
+            wy[e] = e < ny ? my.w[y0 + e] : 0;
+        }
+        for (int qz = mz.ptr[c3]; qz < mz.ptr[c3 + 1]; qz++) {
+            const double wz = mz.w[qz];
+            const double *r = F.r + (long)mz.idx[qz] * fnxy;
+            double v[kHeatList][kHeatList];
+#pragma unroll
+            for (int p = 0; p < kHeatList; p++)
+#pragma unroll
+                for (int q = 0; q < kHeatList; q++) v[p][q] = p < nx && q < ny ? r[(long)ix[p] * F.ny + iy[q]] : 0;
+#pragma unroll
+            for (int p = 0; p < kHeatList; p++)
+#pragma unroll
+                for (int q = 0; q < kHeatList; q++)
+                    if (p < nx && q < ny) {
+                        const double swt = wx[p] * wy[q] * wz;
+                        num += v[p][q] * swt;
+                        den += swt;
+                    }
+        }
+    } else {
+        for (int qz = mz.ptr[c3]; qz < mz.ptr[c3 + 1]; qz++) {
+            const double wz = mz.w[qz];
+            const long oz = (long)mz.idx[qz] * fnxy;
+            for (int qx = x0; qx < x0 + nx; qx++) {
+                const double wx = mx.w[qx];
+                const long ox = oz + (long)mx.idx[qx] * F.ny;
+                for (int qy = y0; qy < y0 + ny; qy++) {
+                    const double swt = wx * my.w[qy] * wz;
+                    num += F.r[ox + my.idx[qy]] * swt;
+                    den += swt;
+                }
             }
         }
     }
@@ -724,6 +853,8 @@ void Solver::heat_set_bc(const int *bondm, long bondm_len, const float *bondv1, 
     heat.nblk = (int)hb(n0);
     heat.partial = (double *)heat_arena.alloc(sizeof(double) * 4 * heat.nblk);
     heat.scal = (double *)heat_arena.alloc(sizeof(double) * 8);
+    heat.count = (unsigned *)heat_arena.alloc(sizeof(unsigned) * 2);
+    P2_CUDA_TRY(cudaMemsetAsync(heat.count, 0, sizeof(unsigned) * 2, st));
     heat.S0 = (double *)heat_arena.alloc(sizeof(double) * n0);
     heat.S1 = (double *)heat_arena.alloc(sizeof(double) * n0);
     {
@@ -738,7 +869,7 @@ void Solver::heat_set_bc(const int *bondm, long bondm_len, const float *bondv1, 
     }
     heat.stage = std::make_shared<HostStage>();
     heat.stage->reserve();
-    P2_CUDA_TRY(cudaMallocHost((void **)&heat.host, sizeof(double) * 8));  // [0..3] error, range; [4] sub-step
+    P2_CUDA_TRY(cudaMallocHost((void **)&heat.host, sizeof(double) * 8));  // [0..3] error, range; [4] sub-step; [6] marker range; [7] barrier
     heat.host_owner.reset(heat.host, [](double *p) { cudaFreeHost(p); });
     P2_CUDA_TRY(cudaStreamSynchronize(st));
     heat.ready = true;
@@ -759,16 +890,52 @@ static HeatLv heat_view(const Level &Lv, const HeatLevel &H, const HeatState &S,
 
 static HeatBc heat_bc_view(const HeatLevel &H) { return HeatBc{H.nbc, H.bu, H.bt, H.bk, H.bconst, H.bpass}; }
 
-void Solver::heat_smooth(int l, int sweeps, double t0koef)
+// The sweeps of a smoothing call, and the residual where the next kernel restricts it.
+void Solver::heat_smooth(int l, int sweeps, double t0koef, bool resid)
 {
     const HeatLv V = heat_view(L[l], heat.lv[l], heat, l);
     const HeatBc B = heat_bc_view(heat.lv[l]);
-    const long half = (long)((V.ny + 1) / 2) * V.nx * V.nz;
+    const long half = V.nh;
+    if (sweeps > 0) {
+        // one block while a thread per node of a colour and per boundary row fits, then a cluster (its barrier
+        // is the cheaper one), then a block per SM: each form is the fastest where it fits (k_heat_sweeps);
+        // a larger level's coefficients do not fit the registers, and it takes a launch per colour
+        const long need = std::max(half, (long)B.nbc), most = kHeatThreads;
+        const int form = need <= most ? kHeatBlock : need <= most * kHeatClusterSize ? kHeatCluster : kHeatGrid;
+        if (need <= most * sm_count) {
+            const long blocks = form == kHeatBlock ? 1 : form == kHeatCluster ? kHeatClusterSize
+                                                       : std::min((long)sm_count, (need + 255) / 256);
+            const GridBarrier S{heat.count, heat.scal + 7};
+            auto kern = form == kHeatBlock ? k_heat_sweeps<kHeatBlock>
+                        : form == kHeatCluster ? k_heat_sweeps<kHeatCluster> : k_heat_sweeps<kHeatGrid>;
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            cfg.gridDim = dim3((unsigned)blocks);
+            cfg.blockDim = dim3((unsigned)(((need + blocks - 1) / blocks + 31) / 32 * 32));
+            cfg.stream = st;
+            cfg.attrs = attr;
+            cfg.numAttrs = form != kHeatBlock;
+            if (form == kHeatCluster) {
+                // the same value from every thread: the attribute belongs to the function, not to this context
+                P2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = (unsigned)blocks;
+                attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            } else {
+                attr[0].id = cudaLaunchAttributeCooperative;
+                attr[0].val.cooperative = 1;
+            }
+            P2_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, V, B, sweeps, t0koef, (int)(l == 0), (int)resid, S));
+            heat.kernels++;
+            return;
+        }
+    }
     for (int s = 0; s < sweeps; s++)
         for (int c = 0; c < 2; c++) {
             k_heat_gs<<<hb(half + B.nbc), 256, 0, st>>>(V, B, c, t0koef, l == 0);
             heat.kernels++;
         }
+    if (!resid) return;
     k_heat_resid<<<hb(V.n), 256, 0, st>>>(V, B, l == 0);
     heat.kernels++;
 }
@@ -781,21 +948,21 @@ void Solver::heat_batch(const p2_heat_params &hp)
     for (int c = 0; c < hp.multicyct; c++) {
         if (nt > 0) {
             for (int l = 0; l < nt; l++) {
-                heat_smooth(l, hp.multittt[0][l], hp.t0koef);
+                heat_smooth(l, hp.multittt[0][l], hp.t0koef, true);
                 const HeatLv F = heat_view(L[l], heat.lv[l], heat, l), C = heat_view(L[l + 1], heat.lv[l + 1], heat, l + 1);
                 const AxisMap *m = heat.lv[l].map;
-                k_heat_restrict<<<hb(C.n), 256, 0, st>>>(F, C, m[0], m[1], m[2]);
+                k_heat_restrict<<<hb(C.n, 128), 128, 0, st>>>(F, C, m[0], m[1], m[2]);
                 heat.kernels++;
             }
             for (int l = nt; l > 0; l--) {
-                heat_smooth(l, hp.multittt[1][l], hp.t0koef);
+                heat_smooth(l, hp.multittt[1][l], hp.t0koef, false);
                 const HeatLv F = heat_view(L[l - 1], heat.lv[l - 1], heat, l - 1), C = heat_view(L[l], heat.lv[l], heat, l);
                 const AxisMap *m = heat.lv[l - 1].map;
                 k_heat_prolong<<<hb(F.n), 256, 0, st>>>(F, C, m[0], m[1], m[2], hp.t1koef);
                 heat.kernels++;
             }
         } else {
-            heat_smooth(0, hp.multittt[0][0], hp.t0koef);
+            heat_smooth(0, hp.multittt[0][0], hp.t0koef, false);
         }
     }
     const HeatLv V0 = heat_view(L[0], heat.lv[0], heat, 0);
@@ -967,9 +1134,13 @@ p2_heat_info Solver::titerate(const p2_heat_params &hp, double timestep, float *
         do {
             P2_CUDA_TRY(cudaGraphLaunch(batch.exec, st));
             heat.kernels += batch.kernels;
-            P2_CUDA_TRY(cudaMemcpyAsync(heat.host, heat.scal, sizeof(double) * 4, cudaMemcpyDeviceToHost, st));
+            P2_CUDA_TRY(cudaMemcpyAsync(heat.host, heat.scal, sizeof(double) * 8, cudaMemcpyDeviceToHost, st));
             P2_CUDA_TRY(cudaStreamSynchronize(st));
             P2_CUDA_TRY(cudaGetLastError());
+            if (heat.host[7] != 0) {
+                P2_CUDA_TRY(cudaMemsetAsync(heat.count, 0, sizeof(unsigned) * 2, st));
+                throw Error(P2_ERR_CUDA, "heat smoother: blocks did not meet at their barrier in time");
+            }
             heatsum = pow(heat.host[0] / heat.host[1], 0.5);
             info.mintk = heat.host[2];
             info.maxtk = heat.host[3];

@@ -19,6 +19,7 @@
 // launch: eight solves at once take 74.6 ms with it, 71.8 ms with clusters only.
 #pragma once
 
+#include "p2_barrier.cuh"
 #include "p2_kernels.cuh"
 
 namespace p2 {
@@ -26,7 +27,6 @@ namespace p2 {
 constexpr int kResThreads = 512;              // two colours of kResSlots cells
 constexpr int kResSlots = kResThreads / 2;
 constexpr int kResCluster = 16;
-constexpr unsigned kResSpin = 1u << 22;       // polls of the grid barrier before it gives up (seconds)
 
 // Boundary rows for the resident sweeps: the rows' chains as for
 // k_bc_set_chain, and per colour and slot the rows that follow one of the
@@ -39,11 +39,6 @@ struct ResidentBC {
     const int *ptr;
     const int4 *dep;
     int cap;  // most entries of one block
-};
-
-struct GridBarrier {
-    unsigned *count;  // [0] arrivals, [1] blocks done; both 0 between launches
-    double *error;    // set to 1 when a wait ran out
 };
 
 struct LoadPlain {
@@ -73,29 +68,6 @@ __host__ __device__ constexpr size_t res_smem(int threads, int tab, int cap)
 {
     return (sizeof(T) * (res_values<kFull>() + 7) + sizeof(float) * kCellEta) * (size_t)threads +
            sizeof(T) * 12 * (size_t)tab + sizeof(ResDep<T>) * (size_t)cap;
-}
-
-// Barrier over the cluster or the whole grid; false when the wait ran out.
-template <bool kCluster>
-__device__ __forceinline__ bool res_sync(GridBarrier B, unsigned &target, bool *ok)
-{
-    if (kCluster) {
-        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
-        return true;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        target += gridDim.x;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(B.count) : "memory");
-        unsigned v = 0, spins = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(B.count) : "memory");
-        } while ((int)(v - target) < 0 && ++spins < kResSpin);
-        *ok = (int)(v - target) >= 0;
-        if (!*ok) *B.error = 1.0;
-    }
-    __syncthreads();
-    return *ok;
 }
 
 template <typename T, bool kFull, bool kCluster>
@@ -289,14 +261,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_smooth_resident(LevelView<T>
         swap(i0, o0); swap(i1, o1); swap(i2, o2); swap(i3, o3);
         if (s + 1 < passes) go = res_sync<kCluster>(B, target, &ok);
     }
-    if (!kCluster && threadIdx.x == 0) {
-        // the last block to leave clears the counters for the next launch
-        __threadfence();
-        if (atomicAdd(B.count + 1, 1u) == gridDim.x - 1) {
-            B.count[0] = 0;
-            B.count[1] = 0;
-        }
-    }
+    if (!kCluster) res_leave(B);
 }
 
 }  // namespace p2

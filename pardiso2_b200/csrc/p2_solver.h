@@ -104,6 +104,7 @@ struct HeatState {
     float *se[12] = {};
     int nblk = 0;
     double *partial = nullptr, *scal = nullptr, *S0 = nullptr, *S1 = nullptr;
+    unsigned *count = nullptr;   // grid barrier counters of the resident sweeps
     double *host = nullptr;
     std::shared_ptr<double> host_owner;
     std::shared_ptr<HostStage> stage;  // pageable arrays of a call
@@ -254,7 +255,7 @@ class Solver {
     void reserve_move_positions(long nmark);
     void velocity_f32();
 
-    void heat_smooth(int l, int sweeps, double t0koef);
+    void heat_smooth(int l, int sweeps, double t0koef, bool resid);
     void heat_batch(const p2_heat_params &hp);
 
     DeviceArena arena, grid_arena, marker_arena, move_arena, post_arena, heat_arena, heat_mk_arena;
