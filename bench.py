@@ -8,10 +8,10 @@ cell (134 M markers), seed 5.  Inputs are seeded synthetic data of those
 shapes (no public dataset exists).
 
 One step = one complete Stokes solve (coarse viscosities, cell factors,
-coarsest LU and inverse, FP64 outer GCR iterations whose preconditioner is
+coarsest inverse, FP64 outer GMRES iterations whose preconditioner is
 one FP32 V-cycle) from a zero initial guess
 on node fields resident in HBM, to ||b - Ax|| / ||b|| <= 1e-8 in FP64.  The
-line also reports the plain FP64 solve (FP64 GCR, FP64 V-cycle), the
+line also reports the plain FP64 solve (FP64 GMRES, FP64 V-cycle), the
 relative L2 error of each field against the FP64 GPU solve and against the
 oracle port's converged solution, the end-to-end host-array call, one RK4
 marker advection step, one heat-equation step, and the oracle port on the
@@ -93,7 +93,7 @@ def parse():
     ap.add_argument("--heat-only", action="store_true",
                     help="only the heat-equation step on the workload's grid, with seeded velocities and "
                          "stresses instead of a solve (profiling runs)")
-    ap.add_argument("--restart", type=int, default=16, help="GCR restart length")
+    ap.add_argument("--restart", type=int, default=16, help="GMRES restart length")
     ap.add_argument("--smoother", type=int, default=1,
                     help="smoother when --tune-iters 0 (profiling runs; the default run autotunes)")
     ap.add_argument("--sweep-growth", type=int, default=2, help="sweep growth per level when --tune-iters 0")
@@ -677,7 +677,7 @@ def main():
         return
     sol = prob.ctx.solution(n)
 
-    # the plain FP64 solve (FP64 GCR, FP64 V-cycle) for comparison; fewer
+    # the plain FP64 solve (FP64 GMRES, FP64 V-cycle) for comparison; fewer
     # steps on the large grids (each is about a second there)
     # the FP64 solve gets its own autotuned schedule (the same candidates),
     # so each precision runs its best configuration
@@ -760,13 +760,13 @@ def main():
     line = {
         "metric": METRIC, "value": value, "unit": "ms", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": False, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f32 V-cycle / f64 outer GCR", "data": "synthetic",
+        "vs_baseline": None, "dtype": "f32 V-cycle / f64 outer GMRES", "data": "synthetic",
         "config": config_dict(args.config, m, world),
         "solver": {"smoother": ("full" if tune.smoother else "diagonal") + " cell-block Vanka, autotuned",
                    "sweeps": "%d pre + %d post on level 0; 4 x %d^l on level l >= 1, at most %d"
                              % (tune.sweeps0, tune.sweeps0, tune.sweep_growth, tune.sweep_max),
-                   "mixed": "FP64 GCR(%d) (true residual and update in FP64), FP32 V-cycle" % tune.restart,
-                   "fp64": "FP64 GCR(%d), FP64 V-cycle, %s cell block, %d + %d sweeps on level 0, 4 x %d^l on level "
+                   "mixed": "FP64 GMRES(%d) (true residual and update in FP64), FP32 V-cycle" % tune.restart,
+                   "fp64": "FP64 GMRES(%d), FP64 V-cycle, %s cell block, %d + %d sweeps on level 0, 4 x %d^l on level "
                            "l >= 1 at most %d (autotuned on its own)"
                            % (tune64.restart, "full" if tune64.smoother else "diagonal", tune64.sweeps0,
                               tune64.sweeps0, tune64.sweep_growth, tune64.sweep_max)},
