@@ -440,6 +440,11 @@ p2_status p2_debug_rows_kernel(p2_ctx *ctx, int variant);
  * solve) applied from zero to the level-0 right-hand side b, both
  * interleaved [P, Vx, Vy, Vz] per node of level 0. */
 p2_status p2_debug_vcycle(p2_ctx *ctx, const double *b, double *x);
+/* The coarsest inverse of the resident node fields alone.  *flag: 0 when the
+ * blocked elimination's inverse stands, otherwise the pivoted LU took its
+ * place; pivoted != 0 takes the LU in any case.  *ms: device time of the way
+ * taken (the first call on a context also captures graphs). */
+p2_status p2_debug_coarse(p2_ctx *ctx, int pivoted, int *flag, double *ms);
 
 #ifdef __cplusplus
 }

@@ -21,7 +21,8 @@ EXPORTED = ["p2_default_params", "p2_create", "p2_destroy", "p2_last_error", "p2
             "p2_set_nodes", "p2_stokes_solve", "p2_stokes_solve_resident", "p2_get_solution", "p2_ronurecalc",
             "p2_upload_markers", "p2_ronurecalc_resident", "p2_get_nodes", "p2_debug_apply", "p2_debug_restrict",
             "p2_debug_prolong", "p2_debug_level_fields", "p2_debug_time_smoother", "p2_debug_smooth",
-            "p2_debug_time_sweep", "p2_debug_time_stage", "p2_debug_rows_kernel", "p2_debug_vcycle", "p2_ronurecalc_noalloc", "p2_autotune",
+            "p2_debug_time_sweep", "p2_debug_time_stage", "p2_debug_rows_kernel", "p2_debug_vcycle", "p2_debug_coarse", "p2_ronurecalc_noalloc",
+            "p2_autotune",
             "p2_movemark", "p2_movemark_resident", "p2_get_markers", "p2_stress_strain",
             "p2_stokes_solve_batch", "p2_movemark_strain", "p2_ronurecalc_powerlaw", "p2_effbulk_visc",
             "p2_default_heat_params", "p2_heat_set_bc", "p2_titerate", "p2_prn_read_header", "p2_prn_read",
@@ -424,9 +425,10 @@ def _debug_sigs(L):
     L.p2_debug_time_stage.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_double)]
     L.p2_debug_rows_kernel.argtypes = [C.c_void_p, C.c_int]
     L.p2_debug_vcycle.argtypes = [C.c_void_p, _dpp, _dpp]
+    L.p2_debug_coarse.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_double)]
     for f in ("p2_debug_apply", "p2_debug_restrict", "p2_debug_prolong", "p2_debug_level_fields",
               "p2_debug_time_smoother", "p2_debug_smooth", "p2_debug_time_sweep", "p2_debug_time_stage",
-              "p2_debug_rows_kernel", "p2_debug_vcycle"):
+              "p2_debug_rows_kernel", "p2_debug_vcycle", "p2_debug_coarse"):
         getattr(L, f).restype = C.c_int
 
 
@@ -491,6 +493,14 @@ class DebugHooks:
         self.ctx._check(self.ctx.L.p2_debug_vcycle(self.ctx.h, np.ascontiguousarray(b, np.float64), x),
                         "p2_debug_vcycle")
         return x
+
+    def coarse(self, pivoted: bool = False):
+        """The coarsest inverse alone: (flag of the blocked elimination, 0 when
+        it stands; ms of the way taken) (p2_debug_coarse)."""
+        flag, ms = C.c_int(), C.c_double()
+        self.ctx._check(self.ctx.L.p2_debug_coarse(self.ctx.h, 1 if pivoted else 0, C.byref(flag), C.byref(ms)),
+                        "p2_debug_coarse")
+        return flag.value, ms.value
 
     def level_fields(self, total_nodes: int):
         nu = np.zeros(total_nodes, np.float32)

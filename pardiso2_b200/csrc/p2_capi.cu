@@ -546,6 +546,15 @@ p2_status p2_debug_vcycle(p2_ctx *ctx, const double *b, double *x)
     });
 }
 
+p2_status p2_debug_coarse(p2_ctx *ctx, int pivoted, int *flag, double *ms)
+{
+    return guard(ctx, [&] {
+        if (!flag || !ms) throw p2::Error(P2_ERR_ARG, "null argument");
+        P2_CUDA_TRY(cudaSetDevice(ctx->s->dev));
+        *flag = ctx->s->debug_coarse(pivoted, ms);
+    });
+}
+
 p2_status p2_debug_time_stage(p2_ctx *ctx, int stage, int level, int variant, int reps, double *ms)
 {
     return guard(ctx, [&] {

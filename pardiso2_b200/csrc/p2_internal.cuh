@@ -42,7 +42,7 @@ struct LuGraph {
     cudaGraphExec_t exec = nullptr;
     int n = 0, kl = -1, ku = -1;
     const double *A = nullptr, *Ainv = nullptr;
-    const int *ipiv = nullptr, *info = nullptr, *perm = nullptr;
+    const int *ipiv = nullptr, *info = nullptr;
     long long kernels = 0;
 };
 

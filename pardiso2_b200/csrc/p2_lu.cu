@@ -698,19 +698,16 @@ static void gj_issue(cudaStream_t st, const double *A, const GjPlan &P, double *
 
 size_t gj_work_doubles(int n) { return (size_t)2 * kGT * n + 4 * kGT * kGT + n; }
 
-// gj_issue replayed as one graph, captured again only when the plan or the
-// buffers change.
+// gj_issue replayed as one graph.  The capture holds the plan and every buffer;
+// the caller drops it with them (a key of sizes and addresses would not do: a
+// freed buffer's address comes back).
 void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
                 LuGraph *cache)
 {
     // per-device attributes, set on the current device (host-side calls)
     P2_CUDA_TRY(cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
     P2_CUDA_TRY(cudaFuncSetAttribute(k_gj_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
-    const bool hit = cache->exec && cache->n == P.n && cache->A == A && cache->Ainv == X && cache->info == d_flag &&
-                     cache->perm == P.perm;
-    if (!hit) {
-        if (cache->exec) cudaGraphExecDestroy(cache->exec);
-        cache->exec = nullptr;
+    if (!cache->exec) {
         cudaGraph_t graph;
         const long long before = g_launches;
         P2_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -721,7 +718,6 @@ void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, fl
         const cudaError_t e = cudaGraphInstantiate(&cache->exec, graph, 0);
         cudaGraphDestroy(graph);
         P2_CUDA_TRY(e);
-        cache->n = P.n; cache->A = A; cache->Ainv = X; cache->info = d_flag; cache->perm = P.perm;
     }
     P2_CUDA_TRY(cudaGraphLaunch(cache->exec, st));
     g_launches += cache->kernels;

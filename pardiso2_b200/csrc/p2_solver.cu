@@ -258,8 +258,7 @@ Solver::~Solver()
     cudaSetDevice(dev);
     if (st_lu) cudaStreamSynchronize(st_lu);
     drop_graphs();
-    if (lu_graph.exec) cudaGraphExecDestroy(lu_graph.exec);
-    if (lu_graph_pivoted.exec) cudaGraphExecDestroy(lu_graph_pivoted.exec);
+    drop_inverse_graphs();
     arena.release();
     grid_arena.release();
     marker_arena.release();
@@ -284,6 +283,17 @@ void Solver::drop_graphs()
     for (auto &g : graphs_apx) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
         g.exec = nullptr;
+    }
+}
+
+// The inverse's graphs hold the plan of the coarsest level (its sizes, tiles and
+// buffers), so they go with it.
+void Solver::drop_inverse_graphs()
+{
+    if (st_lu) cudaStreamSynchronize(st_lu);
+    for (LuGraph *g : {&lu_graph, &lu_graph_pivoted}) {
+        if (g->exec) cudaGraphExecDestroy(g->exec);
+        g->exec = nullptr;
     }
 }
 
@@ -320,6 +330,7 @@ void Solver::set_grid(long nx, long ny, long nz, const double *gx, const double 
     if (p.multinum < 0 || p.multinum + 1 > P2_MAX_LEVELS) throw Error(P2_ERR_ARG, "multinum out of range");
     if (p.p2koef != 0.0) throw Error(P2_ERR_UNSUPPORTED, "p2koef != 0 (grad-div term) is not supported");
     drop_graphs();
+    drop_inverse_graphs();
     arena.release();
     // The cell-block smoothers load the neighbour cells of every cell,
     // including the cell layer above the top one (its values are masked,
@@ -422,6 +433,7 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
     if (!grid_ready) throw Error(P2_ERR_STATE, "p2_set_bc before p2_set_grid");
     if (bondm_len < 4 * total_nodes) throw Error(P2_ERR_ARG, "bondm shorter than 4 * (sum of level nodes)");
     drop_graphs();
+    drop_inverse_graphs();
     arena.release();
     for (size_t l = 0; l < L.size(); l++) {
         Level &Lv = L[l];
@@ -971,11 +983,9 @@ void Solver::lu_pivoted()
 }
 
 // The overlapped inverse: wait for it, order the solve's stream after it and
-// look at its flag; an inverse that failed its check is done again with
-// pivoting.
-void Solver::lu_finish()
+// return its flag.
+int Solver::inverse_flag()
 {
-    if (!lu_pending) return;
     P2_CUDA_TRY(cudaEventSynchronize(ev_lu));
     int flag = 0;
     P2_CUDA_TRY(cudaMemcpyAsync(&flag, d_info, sizeof(int), cudaMemcpyDeviceToHost, st_lu));
@@ -983,7 +993,13 @@ void Solver::lu_finish()
     P2_CUDA_TRY(cudaStreamWaitEvent(st, ev_lu, 0));
     lu_pending = false;
     if (verbose) std::fprintf(stderr, "p2cuda: coarsest inverse n %d (padded %d) flag %d\n", nF, gj.n, flag);
-    if (flag) lu_pivoted();
+    return flag;
+}
+
+// An inverse that failed its check is done again with pivoting.
+void Solver::lu_finish()
+{
+    if (lu_pending && inverse_flag()) lu_pivoted();
 }
 
 // Stand-in for the coarsest direct solve: x = 0, then sweeps of the diagonal
@@ -1970,6 +1986,29 @@ void Solver::debug_vcycle(const double *b, double *x)
     }
     P2_CUDA_TRY(cudaGetLastError());
     from_vec4(st, X.v, L0.n, x);
+}
+
+// The coarsest inverse of the node fields alone: the flag of the blocked
+// elimination (0: it stands, otherwise the pivoted LU takes its place) and the
+// device time in ms of the way taken last; pivoted: the LU in any case.  The
+// first call on a context also captures the graphs.
+int Solver::debug_coarse(int pivoted, double *ms)
+{
+    debug_prepare();
+    coarse_setup();
+    P2_CUDA_TRY(cudaEventRecord(ev[5], st));
+    P2_CUDA_TRY(cudaEventRecord(ev[6], st_lu));
+    const int flag = inverse_flag();
+    if (pivoted || flag) {
+        P2_CUDA_TRY(cudaEventRecord(ev[5], st_lu));
+        lu_pivoted();
+        P2_CUDA_TRY(cudaEventRecord(ev[6], st_lu));
+    }
+    P2_CUDA_TRY(cudaEventSynchronize(ev[6]));
+    float t = 0;
+    P2_CUDA_TRY(cudaEventElapsedTime(&t, ev[5], ev[6]));
+    *ms = t;
+    return flag;
 }
 
 // Average device time of one smoother sweep on level l as the V-cycle runs

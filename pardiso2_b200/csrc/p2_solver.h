@@ -165,6 +165,7 @@ class Solver {
     void drop_graphs_public() { drop_graphs(); }
     void debug_smooth(int level, int sweeps, const double *b, double *x);
     void debug_vcycle(const double *b, double *x);
+    int debug_coarse(int pivoted, double *ms);
     p2_tune_info autotune(int trial_iters);
     bool verbose = false;
 
@@ -210,6 +211,7 @@ class Solver {
     template <typename T>
     LevelView<T> view(int l, bool raw_clamp) const;
     void drop_graphs();
+    void drop_inverse_graphs();
     void allocate_work();
     void build_coarse_index();
     void coarse_setup();
@@ -270,6 +272,7 @@ class Solver {
     int coarse_mode = 0;  // 0: exact coarsest solve (inverse), 1: smoothing sweeps
     int lu_overlap_iters = 0;
     void lu_finish();
+    int inverse_flag();
     template <typename T>
     void coarse_approx(Vec4<T> &b, Vec4<T> &x);
     LuGraph lu_graph;  // coarsest LU + inverse launch sequence
