@@ -445,6 +445,10 @@ p2_status p2_debug_vcycle(p2_ctx *ctx, const double *b, double *x);
  * place; pivoted != 0 takes the LU in any case.  *ms: device time of the way
  * taken (the first call on a context also captures graphs). */
 p2_status p2_debug_coarse(p2_ctx *ctx, int pivoted, int *flag, double *ms);
+/* *in_place: 1 when p2_movemark would move the host array of count floats at p
+ * where it is (one page-locked range holds all of it), 0 when it would copy
+ * it.  Nothing is read or launched. */
+p2_status p2_debug_mapped(p2_ctx *ctx, const void *p, long count, int *in_place);
 
 #ifdef __cplusplus
 }

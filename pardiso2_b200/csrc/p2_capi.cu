@@ -555,6 +555,15 @@ p2_status p2_debug_coarse(p2_ctx *ctx, int pivoted, int *flag, double *ms)
     });
 }
 
+p2_status p2_debug_mapped(p2_ctx *ctx, const void *p, long count, int *in_place)
+{
+    return guard(ctx, [&] {
+        if (!p || !in_place || count < 1) throw p2::Error(P2_ERR_ARG, "null or empty argument");
+        P2_CUDA_TRY(cudaSetDevice(ctx->s->dev));
+        *in_place = p2::movemark_in_place((const float *)p, count);
+    });
+}
+
 p2_status p2_debug_time_stage(p2_ctx *ctx, int stage, int level, int variant, int reps, double *ms)
 {
     return guard(ctx, [&] {

@@ -9,6 +9,7 @@
 //      index and accumulated in that order with the reference's arithmetic
 //      (float accumulators, double weights, no fused multiply-add), so the
 //      node fields equal those of the reference run on one thread.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -816,21 +817,51 @@ void Solver::velocity_f32()
                                              mv_vel[1], mv_vel[2]); P2_COUNT_LAUNCH();
 }
 
-// The device's address of a host array whose whole range is page-locked and
-// mapped, else null.
+// The allocation or registration that holds the device address p; false where
+// the driver names none.
+static bool address_range(const void *p, uintptr_t &start, size_t &size)
+{
+    using Get = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    CUdeviceptr s = 0;
+    size_t n = 0;
+    if (((Get)fn)(&s, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p) != CUDA_SUCCESS ||
+        ((Get)fn)(&n, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) != CUDA_SUCCESS)
+        return false;
+    start = (uintptr_t)s;
+    size = n;
+    return true;
+}
+
+// The device's address of a host array that one page-locked, mapped range
+// holds as a whole, else null.  (Its two ends alone say nothing: two
+// registrations may have pageable memory between them.)  Kernels want it
+// aligned for its type, which a copy did not.
 template <typename V>
 static V *mapped(V *p, long n)
 {
-    const char *lo = (const char *)p, *hi = (const char *)(p + n) - 1;
-    cudaPointerAttributes a, b;
-    if (cudaPointerGetAttributes(&a, lo) != cudaSuccess || cudaPointerGetAttributes(&b, hi) != cudaSuccess) {
+    const size_t bytes = sizeof(V) * (size_t)n;
+    cudaPointerAttributes a;
+    if ((uintptr_t)p % alignof(V) || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer) return nullptr;
-    if ((const char *)b.devicePointer - (const char *)a.devicePointer != hi - lo) return nullptr;
+    if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+    uintptr_t start = 0;
+    size_t size = 0;
+    const uintptr_t d = (uintptr_t)a.devicePointer;
+    if (!address_range(a.devicePointer, start, size) || d < start || d - start > size || bytes > size - (d - start))
+        return nullptr;
     return (V *)a.devicePointer;
 }
+
+bool movemark_in_place(const float *p, long n) { return mapped(p, n) != nullptr; }
 
 // movemark() on host arrays: velocities vx, vy, vz (float, node layout) and
 // markers in/out.

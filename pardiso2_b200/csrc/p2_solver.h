@@ -118,6 +118,9 @@ struct HeatState {
     long long kernels = 0;
 };
 
+// whether p2_movemark moves a host array of n floats where it is (debug hook)
+bool movemark_in_place(const float *p, long n);
+
 class Solver {
   public:
     explicit Solver(int device);
