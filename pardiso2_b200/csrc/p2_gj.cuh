@@ -162,10 +162,11 @@ __device__ __forceinline__ void gj_invert(const double *sh, double *w, double *D
     }
 }
 
-// X = A in the permuted order with identity padding, column-major n x n
+// X = A in the permuted order with identity padding, column-major n x n; the
+// columns along the grid's x, whose y ends at 65535
 __global__ void k_gj_gather(int n, int nF, const int *perm, const double *A, double *X)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    const int r = blockIdx.y * blockDim.x + threadIdx.x, c = blockIdx.x;
     if (r >= n) return;
     const int pr = perm[r], pc = perm[c];
     double v = r == c ? 1.0 : 0.0;

@@ -1120,13 +1120,9 @@ p2_heat_info Solver::titerate(const p2_heat_params &hp, double timestep, float *
         if (!batch.exec) {
             // multicyct V-cycles and the error reduction as one graph
             const long long k0 = heat.kernels;
-            cudaGraph_t g = nullptr;
-            P2_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            Capture capture(st);
             heat_batch(hp);
-            P2_CUDA_TRY(cudaStreamEndCapture(st, &g));
-            const cudaError_t e = cudaGraphInstantiate(&batch.exec, g, 0);
-            cudaGraphDestroy(g);
-            P2_CUDA_TRY(e);
+            capture.instantiate(&batch.exec);
             batch.kernels = heat.kernels - k0;
             heat.kernels = k0;
         }

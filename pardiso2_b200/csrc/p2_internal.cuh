@@ -79,6 +79,39 @@ struct Error {
     Error(p2_status c, std::string m) : code(c), msg(std::move(m)) {}
 };
 
+// A stream capture that ends with its scope: an error thrown between begin and
+// end would otherwise leave the stream capturing, and every later call on it
+// would fail.
+class Capture {
+  public:
+    explicit Capture(cudaStream_t s) : st(s)
+    {
+        P2_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        open = true;
+    }
+    ~Capture()
+    {
+        if (open) {
+            cudaStreamEndCapture(st, &graph);
+            cudaGetLastError();
+        }
+        if (graph) cudaGraphDestroy(graph);
+    }
+    Capture(const Capture &) = delete;
+    Capture &operator=(const Capture &) = delete;
+    void instantiate(cudaGraphExec_t *exec)
+    {
+        open = false;
+        P2_CUDA_TRY(cudaStreamEndCapture(st, &graph));
+        P2_CUDA_TRY(cudaGraphInstantiate(exec, graph, 0));
+    }
+
+  private:
+    cudaStream_t st;
+    cudaGraph_t graph = nullptr;
+    bool open = false;
+};
+
 // Bits of the per-node boundary mask: bit c set when unknown (node, c) is a
 // boundary row (c = 0 P, 1 Vx, 2 Vy, 3 Vz).  The pinned pressure cell is not
 // marked: it is smoothed as a continuity row and fixed by a pressure shift.

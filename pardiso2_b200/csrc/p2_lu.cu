@@ -642,16 +642,12 @@ int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *A
         if (!hit) {
             if (cache->exec) cudaGraphExecDestroy(cache->exec);
             cache->exec = nullptr;
-            cudaGraph_t graph;
             long long before = g_launches;
-            P2_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            Capture capture(st);
             lu_issue(st, A, n, kl, ku, Ainv, d_ipiv, d_info, T);
-            P2_CUDA_TRY(cudaStreamEndCapture(st, &graph));
             cache->kernels = g_launches - before;
             g_launches = before;
-            cudaError_t e = cudaGraphInstantiate(&cache->exec, graph, 0);
-            cudaGraphDestroy(graph);
-            P2_CUDA_TRY(e);
+            capture.instantiate(&cache->exec);
             cache->n = n; cache->kl = kl; cache->ku = ku; cache->A = A; cache->Ainv = Ainv;
             cache->ipiv = d_ipiv; cache->info = d_info;
         }
@@ -681,7 +677,7 @@ static void gj_issue(cudaStream_t st, const double *A, const GjPlan &P, double *
     const int n = P.n, nt = n / kGT;
     double *Lb = work, *Ub = Lb + (size_t)kGT * n, *D = Ub + (size_t)kGT * n, *y = D + 4 * kGT * kGT;
     P2_CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), st));
-    k_gj_gather<<<dim3((n + 255) / 256, n), 256, 0, st>>>(n, P.nF, P.perm, A, X); P2_COUNT_LAUNCH();
+    k_gj_gather<<<dim3(n, (n + 255) / 256), 256, 0, st>>>(n, P.nF, P.perm, A, X); P2_COUNT_LAUNCH();
     k_gj_first<<<1, kGThreads, 0, st>>>(X, n, D, d_flag); P2_COUNT_LAUNCH();
     for (int p = 0; p < nt; p++) {
         const GjTiles T{P.tv[p], P.tq[p], P.nv / kGT};
@@ -708,16 +704,12 @@ void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, fl
     P2_CUDA_TRY(cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
     P2_CUDA_TRY(cudaFuncSetAttribute(k_gj_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
     if (!cache->exec) {
-        cudaGraph_t graph;
         const long long before = g_launches;
-        P2_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        Capture capture(st);
         gj_issue(st, A, P, X, Xf, work, d_flag);
-        P2_CUDA_TRY(cudaStreamEndCapture(st, &graph));
         cache->kernels = g_launches - before;
         g_launches = before;
-        const cudaError_t e = cudaGraphInstantiate(&cache->exec, graph, 0);
-        cudaGraphDestroy(graph);
-        P2_CUDA_TRY(e);
+        capture.instantiate(&cache->exec);
     }
     P2_CUDA_TRY(cudaGraphLaunch(cache->exec, st));
     g_launches += cache->kernels;
@@ -727,14 +719,14 @@ void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, fl
 // in A's order
 __global__ void k_permute_inverse(int n, int nF, const int *perm, const double *B, double *X)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    const int r = blockIdx.y * blockDim.x + threadIdx.x, c = blockIdx.x;
     if (r >= n) return;
     const int pr = perm[r], pc = perm[c];
     X[(size_t)c * n + r] = pr >= 0 && pc >= 0 ? B[(size_t)pc * nF + pr] : (r == c ? 1.0 : 0.0);
 }
 void permute_inverse(cudaStream_t st, const GjPlan &P, const double *B, double *X)
 {
-    k_permute_inverse<<<dim3((P.n + 255) / 256, P.n), 256, 0, st>>>(P.n, P.nF, P.perm, B, X); P2_COUNT_LAUNCH();
+    k_permute_inverse<<<dim3(P.n, (P.n + 255) / 256), 256, 0, st>>>(P.n, P.nF, P.perm, B, X); P2_COUNT_LAUNCH();
     P2_CUDA_TRY(cudaGetLastError());
 }
 

@@ -1436,15 +1436,12 @@ void Solver::capture_vcycle_graph()
 {
     GraphSlot &g = (coarse_mode ? graphs_apx : graphs)[std::is_same<T, double>::value ? 1 : 0];
     if (g.exec || !prm.use_graphs) return;
-    cudaGraph_t graph;
     long long before = g_launches;
-    P2_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    Capture capture(st);
     vcycle<T>();
-    P2_CUDA_TRY(cudaStreamEndCapture(st, &graph));
     g.kernels = g_launches - before;  // captured, not yet executed
     g_launches = before;
-    P2_CUDA_TRY(cudaGraphInstantiate(&g.exec, graph, 0));
-    cudaGraphDestroy(graph);
+    capture.instantiate(&g.exec);
     P2_CUDA_TRY(cudaGraphUpload(g.exec, st));
 }
 
