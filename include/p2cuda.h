@@ -440,11 +440,12 @@ p2_status p2_debug_rows_kernel(p2_ctx *ctx, int variant);
  * solve) applied from zero to the level-0 right-hand side b, both
  * interleaved [P, Vx, Vy, Vz] per node of level 0. */
 p2_status p2_debug_vcycle(p2_ctx *ctx, const double *b, double *x);
-/* The coarsest inverse of the resident node fields alone.  *flag: 0 when the
- * blocked elimination's inverse stands, otherwise the pivoted LU took its
- * place; pivoted != 0 takes the LU in any case.  *ms: device time of the way
- * taken (the first call on a context also captures graphs). */
-p2_status p2_debug_coarse(p2_ctx *ctx, int pivoted, int *flag, double *ms);
+/* The coarsest inverse of the resident node fields alone.  way: 0 the one a
+ * solve takes, by the level's sizes; 1 the pivoted LU; 2 the blocked
+ * elimination.  *flag: -1 when the LU was taken from the start, otherwise 0
+ * when the blocked inverse stands, else the LU took its place.  *ms: its
+ * device time (the first call on a context also captures graphs). */
+p2_status p2_debug_coarse(p2_ctx *ctx, int way, int *flag, double *ms);
 /* *in_place: 1 when p2_movemark would move the host array of count floats at p
  * where it is (one page-locked range holds all of it), 0 when it would copy
  * it.  Nothing is read or launched. */

@@ -495,11 +495,12 @@ class DebugHooks:
                         "p2_debug_vcycle")
         return x
 
-    def coarse(self, pivoted: bool = False):
-        """The coarsest inverse alone: (flag of the blocked elimination, 0 when
-        it stands; ms of the way taken) (p2_debug_coarse)."""
+    def coarse(self, way: int = 0):
+        """The coarsest inverse alone, by rule (0), pivoted LU (1) or blocked
+        elimination (2): (flag: -1 the LU from the start, 0 the blocked one
+        stands, else the LU took its place; ms) (p2_debug_coarse)."""
         flag, ms = C.c_int(), C.c_double()
-        self.ctx._check(self.ctx.L.p2_debug_coarse(self.ctx.h, 1 if pivoted else 0, C.byref(flag), C.byref(ms)),
+        self.ctx._check(self.ctx.L.p2_debug_coarse(self.ctx.h, way, C.byref(flag), C.byref(ms)),
                         "p2_debug_coarse")
         return flag.value, ms.value
 

@@ -546,12 +546,12 @@ p2_status p2_debug_vcycle(p2_ctx *ctx, const double *b, double *x)
     });
 }
 
-p2_status p2_debug_coarse(p2_ctx *ctx, int pivoted, int *flag, double *ms)
+p2_status p2_debug_coarse(p2_ctx *ctx, int way, int *flag, double *ms)
 {
     return guard(ctx, [&] {
-        if (!flag || !ms) throw p2::Error(P2_ERR_ARG, "null argument");
+        if (!flag || !ms || way < 0 || way > 2) throw p2::Error(P2_ERR_ARG, "null argument or unknown way");
         P2_CUDA_TRY(cudaSetDevice(ctx->s->dev));
-        *flag = ctx->s->debug_coarse(pivoted, ms);
+        *flag = ctx->s->debug_coarse(way, ms);
     });
 }
 

@@ -18,8 +18,8 @@
 // velocities and np pressures.  n = 3648 (12^3 nodes): the full update 74 us,
 // 23 TFLOP/s, the panel 8.5 us, the whole inverse 4.3 ms; the pivoted band LU
 // and its triangular solves, a serial chain of 114 panels in one block, took
-// 13 ms.  The inverse was faster than the band LU at every size measured, from
-// 11^3 (2.8 against 8.5 ms of a solve) to 21^3 nodes on one level.
+// 13 ms.  The LU's work grows with the band instead of n, so large and long
+// levels take it from the start (gj_prefers_lu).
 #pragma once
 
 #include "p2_internal.cuh"

@@ -54,6 +54,7 @@ struct GjPlan {
     int nF = 0, n = 0, nv = 0;  // unknowns, padded size, padded velocity part
     const int *perm = nullptr, *iperm = nullptr;
     std::vector<int> tv, tq;
+    bool lu_first = false;  // the pivoted band LU is the shorter way
 };
 #define P2_COUNT_LAUNCH() (++p2::g_launches)
 

@@ -533,8 +533,8 @@ struct LuTimer {
 };
 
 // Factor the banded A (n x n, column-major, lower/upper half-bandwidths kl,
-// ku) in place and write its inverse into Ainv.  Returns 0 or the first
-// zero-pivot column + 1.
+// ku) in place and write its inverse into Ainv; *d_info: 0 or the first
+// zero-pivot column + 1, once the stream has finished.
 // panels per group in the backward half of the inverse
 constexpr int kInvGroup = 4;
 
@@ -616,8 +616,8 @@ static void lu_issue(cudaStream_t st, double *A, int n, int kl, int ku, double *
     P2_CUDA_TRY(cudaGetLastError());
 }
 
-int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *Ainv, int *d_ipiv, int *d_info,
-                    LuGraph *cache)
+void band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *Ainv, int *d_ipiv, int *d_info,
+                     LuGraph *cache)
 {
     kl = std::max(0, std::min(kl, n - 1));
     ku = std::max(0, std::min(ku, n - 1));
@@ -663,10 +663,6 @@ int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *A
         cudaEventDestroy(T.a);
         cudaEventDestroy(T.b);
     }
-    int info = 0;
-    P2_CUDA_TRY(cudaMemcpyAsync(&info, d_info, sizeof(int), cudaMemcpyDeviceToHost, st));
-    P2_CUDA_TRY(cudaStreamSynchronize(st));
-    return info;
 }
 
 // Inverse of A (nF x nF, column-major) into X (n x n in the plan's order, see

@@ -32,8 +32,8 @@
 namespace p2 {
 
 constexpr int kProbes = 4 * 125;  // coarsest-operator probes: 125 colour classes x 4 components
-int band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *Ainv, int *d_ipiv, int *d_info,
-                    LuGraph *cache);
+void band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *Ainv, int *d_ipiv, int *d_info,
+                     LuGraph *cache);
 // sweeps of the diagonal cell smoother on the coarsest level standing in for
 // its direct solve while the LU is still running
 constexpr int kCoarseApxSweeps = 16;
@@ -55,6 +55,20 @@ size_t gj_work_doubles(int n);
 void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
                 LuGraph *cache);
 void permute_inverse(cudaStream_t st, const GjPlan &P, const double *B, double *X);
+
+// Which inverse of nF unknowns, nv of them velocities, is the shorter one: ms per
+// column of the blocked elimination and of the pivoted LU for a half band of b.
+// Both lines are fits to one-level grids (blocked / LU, ms): 12^3 4.0 / 12.7,
+// 17^3 110 / 198, 21^3 901 / 925, 23^3 2213 / 1759, 27^3 10575 / 5977, 8 x 8 x 60
+// 22 / 24, 8 x 8 x 120 170 / 63, 12 x 12 x 40 139 / 87, 12 x 40 x 12 165 / 375.  The
+// elimination's work grows with the square of the unknowns a column, the LU's with
+// the band, so large and long levels (z is the outermost axis) take the LU.
+static bool gj_prefers_lu(double nF, double nv, double b)
+{
+    const double blocked = 5.4e-4 + 8.9e-11 * nF * (nv / 3 + (nF - nv));
+    const double lu = 1.56e-3 + 3.7e-6 * b + 6.8e-10 * nF * b;
+    return lu < blocked;
+}
 
 static inline unsigned nblk(long n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
 
@@ -839,6 +853,20 @@ void Solver::build_coarse_index()
             gj.tv[p] = std::max(reach(part[0], plane), std::min(p + 2, nvt));
             gj.tq[p] = p + 1 == nvt ? nt - nvt : reach(part[1], plane);
         }
+        // the widest coupling in the natural order, one node on along every axis, as the LU's half band
+        int band = 1;
+        {
+            const int corner = plane_nodes + C.ny + 1;
+            std::vector<int> lo(C.n, -1), hi(C.n, -1);
+            for (int q = 0; q < nF; q++) {
+                const int u = fre[q] >> 2;
+                if (lo[u] < 0) lo[u] = q;
+                hi[u] = q;
+            }
+            for (int u = 0; u + corner < C.n; u++)
+                if (lo[u] >= 0 && hi[u + corner] >= 0) band = std::max(band, hi[u + corner] - lo[u]);
+        }
+        gj.lu_first = gj_prefers_lu(nF, gj.nv, band);
         gj.perm = upload(arena, perm);
         gj.iperm = upload(arena, iperm);
         d_slots = upload(arena, list);
@@ -857,7 +885,6 @@ void Solver::build_coarse_index()
     Ainv64 = (double *)arena.alloc(sizeof(double) * (size_t)gj.n * gj.n);
     Ainv32 = (float *)arena.alloc(sizeof(float) * (size_t)gj.n * gj.n);
     gj_work = (double *)arena.alloc(sizeof(double) * gj_work_doubles(gj.n));
-    Ainv_natural = nullptr;
     d_ipiv = (int *)arena.alloc(sizeof(int) * nF);
     d_info = (int *)arena.alloc(sizeof(int) * 4);
     probes = (double *)arena.alloc(sizeof(double) * (size_t)C.n * 4 * kProbes);
@@ -941,9 +968,10 @@ __global__ void k_probe_rows(LevelView<double> Lc, const double *probes, const i
     }
 }
 
-void Solver::coarse_setup()
+// way: 0 the inverse that the plan's sizes choose, 1 the pivoted LU, 2 the blocked elimination
+void Solver::coarse_setup(int way)
 {
-    // an LU left running by a solve that ended in an error still reads A_c
+    // an inverse left running by a solve that ended in an error still reads A_c
     P2_CUDA_TRY(cudaStreamSynchronize(st_lu));
     lu_pending = false;
     Level &C = L.back();
@@ -959,27 +987,31 @@ void Solver::coarse_setup()
     // coarsest level for lu_overlap_iters outer iterations.
     P2_CUDA_TRY(cudaEventRecord(ev_lu, st));
     P2_CUDA_TRY(cudaStreamWaitEvent(st_lu, ev_lu, 0));
-    gj_inverse(st_lu, A_c, gj, Ainv64, prm.precision == 0 ? Ainv32 : nullptr, gj_work, d_info, &lu_graph);
-    P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
+    lu_pivoted = way == 1 || (way == 0 && gj.lu_first);
+    if (lu_pivoted) {
+        invert_pivoted();
+    } else {
+        gj_inverse(st_lu, A_c, gj, Ainv64, prm.precision == 0 ? Ainv32 : nullptr, gj_work, d_info, &lu_graph);
+        P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
+    }
     lu_pending = true;
     lu_overlap_iters = L.size() < 3 ? 0
                        : (int)std::min<double>(kOverlapMax, kOverlapScale * nF / (double)L[0].n);
 }
 
-// The inverse by the pivoted band LU (A_c is overwritten), brought into the
-// slots' order; its buffer is allocated on first use.
-void Solver::lu_pivoted()
+// The inverse by the pivoted band LU, brought into the slots' order.  It is
+// formed in Ainv64 in A_c's order; A_c, whose factors are then no longer needed,
+// takes it for the permutation, so that no third matrix is held.
+void Solver::invert_pivoted()
 {
     P2_CUDA_TRY(cudaMemcpyAsync(h_bw, d_bw, sizeof(int) * 2, cudaMemcpyDeviceToHost, st_lu));
     P2_CUDA_TRY(cudaStreamSynchronize(st_lu));
-    if (!Ainv_natural) Ainv_natural = (double *)arena.alloc(sizeof(double) * (size_t)nF * nF);
-    const int info = band_lu_inverse(st_lu, A_c, nF, h_bw[0], h_bw[1], Ainv_natural, d_ipiv, d_info, &lu_graph_pivoted);
-    if (info) throw Error(P2_ERR_SINGULAR, "zero pivot in the coarsest LU at column " + std::to_string(info));
-    permute_inverse(st_lu, gj, Ainv_natural, Ainv64);
-    d2f(st_lu, (size_t)gj.n * gj.n, Ainv64, Ainv32);
+    band_lu_inverse(st_lu, A_c, nF, h_bw[0], h_bw[1], Ainv64, d_ipiv, d_info, &lu_graph_pivoted);
+    P2_CUDA_TRY(cudaMemcpyAsync(A_c, Ainv64, sizeof(double) * (size_t)nF * nF, cudaMemcpyDeviceToDevice, st_lu));
+    permute_inverse(st_lu, gj, A_c, Ainv64);
+    if (prm.precision == 0) d2f(st_lu, (size_t)gj.n * gj.n, Ainv64, Ainv32);
     P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
-    P2_CUDA_TRY(cudaStreamWaitEvent(st, ev_lu, 0));
-    lu_pending = false;
+    lu_pivoted = true;
 }
 
 // The overlapped inverse: wait for it, order the solve's stream after it and
@@ -991,15 +1023,26 @@ int Solver::inverse_flag()
     P2_CUDA_TRY(cudaMemcpyAsync(&flag, d_info, sizeof(int), cudaMemcpyDeviceToHost, st_lu));
     P2_CUDA_TRY(cudaStreamSynchronize(st_lu));
     P2_CUDA_TRY(cudaStreamWaitEvent(st, ev_lu, 0));
-    lu_pending = false;
-    if (verbose) std::fprintf(stderr, "p2cuda: coarsest inverse n %d (padded %d) flag %d\n", nF, gj.n, flag);
+    if (verbose)
+        std::fprintf(stderr, "p2cuda: coarsest inverse n %d (padded %d) %s flag %d\n", nF, gj.n,
+                     lu_pivoted ? "pivoted" : "blocked", flag);
     return flag;
 }
 
-// An inverse that failed its check is done again with pivoting.
-void Solver::lu_finish()
+// A blocked inverse that failed its check is done again with pivoting.  Returns
+// the flag of the first inverse.
+int Solver::lu_finish()
 {
-    if (lu_pending && inverse_flag()) lu_pivoted();
+    if (!lu_pending) return 0;
+    const int first = inverse_flag();
+    int flag = first;
+    if (flag && !lu_pivoted) {
+        invert_pivoted();
+        flag = inverse_flag();
+    }
+    lu_pending = false;
+    if (flag) throw Error(P2_ERR_SINGULAR, "zero pivot in the coarsest LU at column " + std::to_string(flag));
+    return first;
 }
 
 // Stand-in for the coarsest direct solve: x = 0, then sweeps of the diagonal
@@ -1985,27 +2028,23 @@ void Solver::debug_vcycle(const double *b, double *x)
     from_vec4(st, X.v, L0.n, x);
 }
 
-// The coarsest inverse of the node fields alone: the flag of the blocked
-// elimination (0: it stands, otherwise the pivoted LU takes its place) and the
-// device time in ms of the way taken last; pivoted: the LU in any case.  The
-// first call on a context also captures the graphs.
-int Solver::debug_coarse(int pivoted, double *ms)
+// The coarsest inverse of the node fields alone (way as for coarse_setup): -1
+// when the pivoted LU was taken from the start, otherwise the flag of the blocked
+// elimination (0: it stands, else the pivoted LU took its place), and its
+// device time in ms.  The first call on a context also captures the graphs.
+int Solver::debug_coarse(int way, double *ms)
 {
     debug_prepare();
-    coarse_setup();
+    coarse_setup(way);
     P2_CUDA_TRY(cudaEventRecord(ev[5], st));
+    const bool pivoted = lu_pivoted;
+    const int flag = lu_finish();
     P2_CUDA_TRY(cudaEventRecord(ev[6], st_lu));
-    const int flag = inverse_flag();
-    if (pivoted || flag) {
-        P2_CUDA_TRY(cudaEventRecord(ev[5], st_lu));
-        lu_pivoted();
-        P2_CUDA_TRY(cudaEventRecord(ev[6], st_lu));
-    }
     P2_CUDA_TRY(cudaEventSynchronize(ev[6]));
     float t = 0;
     P2_CUDA_TRY(cudaEventElapsedTime(&t, ev[5], ev[6]));
     *ms = t;
-    return flag;
+    return pivoted ? -1 : flag;
 }
 
 // Average device time of one smoother sweep on level l as the V-cycle runs

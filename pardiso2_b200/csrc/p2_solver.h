@@ -168,7 +168,7 @@ class Solver {
     void drop_graphs_public() { drop_graphs(); }
     void debug_smooth(int level, int sweeps, const double *b, double *x);
     void debug_vcycle(const double *b, double *x);
-    int debug_coarse(int pivoted, double *ms);
+    int debug_coarse(int way, double *ms);
     p2_tune_info autotune(int trial_iters);
     bool verbose = false;
 
@@ -217,7 +217,7 @@ class Solver {
     void drop_inverse_graphs();
     void allocate_work();
     void build_coarse_index();
-    void coarse_setup();
+    void coarse_setup(int way = 0);
     template <typename T>
     void coarse_solve(Vec4<T> &b, Vec4<T> &x);
     template <typename T>
@@ -274,7 +274,7 @@ class Solver {
     bool lu_pending = false;
     int coarse_mode = 0;  // 0: exact coarsest solve (inverse), 1: smoothing sweeps
     int lu_overlap_iters = 0;
-    void lu_finish();
+    int lu_finish();
     int inverse_flag();
     template <typename T>
     void coarse_approx(Vec4<T> &b, Vec4<T> &x);
@@ -299,9 +299,10 @@ class Solver {
     int *d_colmap = nullptr, *d_crt = nullptr;
     GjPlan gj;
     int *d_slots = nullptr, *d_slot_of = nullptr;  // unknown of each slot of the inverse (-1 padding), and back
-    double *gj_work = nullptr, *Ainv_natural = nullptr;
+    double *gj_work = nullptr;
     LuGraph lu_graph_pivoted;
-    void lu_pivoted();
+    void invert_pivoted();
+    bool lu_pivoted = false;  // the inverse in flight is the pivoted LU's
     float *d_crk = nullptr;
     double *A_c = nullptr, *Ainv64 = nullptr;
     float *Ainv32 = nullptr;
