@@ -446,6 +446,10 @@ p2_status p2_debug_vcycle(p2_ctx *ctx, const double *b, double *x);
  * when the blocked inverse stands, else the LU took its place.  *ms: its
  * device time (the first call on a context also captures graphs). */
 p2_status p2_debug_coarse(p2_ctx *ctx, int way, int *flag, double *ms);
+/* For the following p2_set_bc and p2_heat_set_bc of this context: the forms of
+ * the resident sweeps as on a device that places no cluster of 16 blocks (1),
+ * nor a cooperative grid of a block per SM (2); 0, the default, asks the device. */
+p2_status p2_debug_forms(p2_ctx *ctx, int without);
 /* *in_place: 1 when p2_movemark would move the host array of count floats at p
  * where it is (one page-locked range holds all of it), 0 when it would copy
  * it.  Nothing is read or launched. */

@@ -21,7 +21,7 @@ EXPORTED = ["p2_default_params", "p2_create", "p2_destroy", "p2_last_error", "p2
             "p2_set_nodes", "p2_stokes_solve", "p2_stokes_solve_resident", "p2_get_solution", "p2_ronurecalc",
             "p2_upload_markers", "p2_ronurecalc_resident", "p2_get_nodes", "p2_debug_apply", "p2_debug_restrict",
             "p2_debug_prolong", "p2_debug_level_fields", "p2_debug_time_smoother", "p2_debug_smooth",
-            "p2_debug_time_sweep", "p2_debug_time_stage", "p2_debug_rows_kernel", "p2_debug_vcycle", "p2_debug_coarse", "p2_debug_mapped", "p2_ronurecalc_noalloc",
+            "p2_debug_time_sweep", "p2_debug_time_stage", "p2_debug_rows_kernel", "p2_debug_vcycle", "p2_debug_coarse", "p2_debug_forms", "p2_debug_mapped", "p2_ronurecalc_noalloc",
             "p2_autotune",
             "p2_movemark", "p2_movemark_resident", "p2_get_markers", "p2_stress_strain",
             "p2_stokes_solve_batch", "p2_movemark_strain", "p2_ronurecalc_powerlaw", "p2_effbulk_visc",
@@ -426,10 +426,12 @@ def _debug_sigs(L):
     L.p2_debug_rows_kernel.argtypes = [C.c_void_p, C.c_int]
     L.p2_debug_vcycle.argtypes = [C.c_void_p, _dpp, _dpp]
     L.p2_debug_mapped.argtypes = [C.c_void_p, C.c_void_p, C.c_long, C.POINTER(C.c_int)]
+    L.p2_debug_forms.argtypes = [C.c_void_p, C.c_int]
     L.p2_debug_coarse.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_double)]
     for f in ("p2_debug_apply", "p2_debug_restrict", "p2_debug_prolong", "p2_debug_level_fields",
               "p2_debug_time_smoother", "p2_debug_smooth", "p2_debug_time_sweep", "p2_debug_time_stage",
-              "p2_debug_rows_kernel", "p2_debug_vcycle", "p2_debug_coarse", "p2_debug_mapped"):
+              "p2_debug_rows_kernel", "p2_debug_vcycle", "p2_debug_coarse", "p2_debug_forms",
+              "p2_debug_mapped"):
         getattr(L, f).restype = C.c_int
 
 
@@ -503,6 +505,10 @@ class DebugHooks:
         self.ctx._check(self.ctx.L.p2_debug_coarse(self.ctx.h, way, C.byref(flag), C.byref(ms)),
                         "p2_debug_coarse")
         return flag.value, ms.value
+
+    def forms(self, without: int):
+        """Resident sweeps of later set-ups without clusters (1), without grids too (2) (p2_debug_forms)."""
+        self.ctx._check(self.ctx.L.p2_debug_forms(self.ctx.h, without), "p2_debug_forms")
 
     def mapped(self, address: int, count: int) -> bool:
         """Whether p2_movemark would move `count` floats at a host address in place (p2_debug_mapped)."""

@@ -546,6 +546,14 @@ p2_status p2_debug_vcycle(p2_ctx *ctx, const double *b, double *x)
     });
 }
 
+p2_status p2_debug_forms(p2_ctx *ctx, int without)
+{
+    return guard(ctx, [&] {
+        if (without < 0 || without > 2) throw p2::Error(P2_ERR_ARG, "without must be 0, 1 or 2");
+        ctx->s->dbg_forms = without;
+    });
+}
+
 p2_status p2_debug_coarse(p2_ctx *ctx, int way, int *flag, double *ms)
 {
     return guard(ctx, [&] {

@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256) k_heat_resid(HeatLv L, HeatBc B, int leve
 // a cluster 2.7 / 2.1 (13^3), 2.9 / 2.5 (31 x 33 x 31), the grid 3.0 / 2.8
 // (37^3), 3.7 / 3.3 (65^3); the step on 65^3 nodes 5.6 -> 4.5 ms between its
 // events without markers, 982 -> 232 launches.
-enum { kHeatBlock = 0, kHeatCluster = 1, kHeatGrid = 2 };
+enum { kHeatBlock = 0, kHeatCluster = 1, kHeatGrid = 2, kHeatPasses = 3 };
 constexpr int kHeatThreads = 1024;  // of a block at most: 64 registers each
 constexpr int kHeatClusterSize = 16;
 
@@ -828,6 +828,7 @@ void Solver::heat_set_bc(const int *bondm, long bondm_len, const float *bondv1, 
         H.b = (double *)heat_arena.alloc(sizeof(double) * 2 * nh);
         H.r = (double *)heat_arena.alloc(sizeof(double) * n);
         H.a = (double *)heat_arena.alloc(sizeof(double) * 7 * 2 * nh);
+        heat_choose_form(H);
         P2_CUDA_TRY(cudaMemsetAsync(H.x, 0, sizeof(double) * n, st));
         P2_CUDA_TRY(cudaMemsetAsync(H.b, 0, sizeof(double) * 2 * nh, st));
         if (l > 0) {
@@ -890,45 +891,76 @@ static HeatLv heat_view(const Level &Lv, const HeatLevel &H, const HeatState &S,
 
 static HeatBc heat_bc_view(const HeatLevel &H) { return HeatBc{H.nbc, H.bu, H.bt, H.bk, H.bconst, H.bpass}; }
 
+using HeatSweeps = void (*)(HeatLv, HeatBc, int, double, int, int, GridBarrier);
+
+// The launch of a level's sweeps in its form (not kHeatPasses).  The function
+// attribute is the same from every thread: it belongs to the function, not to
+// this context.
+static cudaError_t heat_config(const HeatLevel &H, HeatSweeps &kern, cudaLaunchConfig_t &cfg, cudaLaunchAttribute attr[1])
+{
+    kern = H.form == kHeatBlock ? k_heat_sweeps<kHeatBlock>
+           : H.form == kHeatCluster ? k_heat_sweeps<kHeatCluster> : k_heat_sweeps<kHeatGrid>;
+    cfg = {};
+    cfg.gridDim = dim3(H.blocks);
+    cfg.blockDim = dim3(H.threads);
+    cfg.attrs = attr;
+    cfg.numAttrs = H.form != kHeatBlock;
+    if (H.form == kHeatCluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = H.blocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    return cudaSuccess;
+}
+
+// One block while a thread per node of a colour and per boundary row fits, then
+// a cluster (its barrier is the cheaper one), then a block per SM: each form is
+// the fastest where it fits (k_heat_sweeps) and is taken where the device can
+// place it; a larger level's coefficients do not fit the registers, and it takes
+// a launch per colour.
+void Solver::heat_choose_form(HeatLevel &H)
+{
+    const long need = std::max(H.nh, (long)H.nbc), most = kHeatThreads;
+    for (H.form = kHeatBlock; H.form < kHeatPasses; H.form++) {
+        const long blocks = H.form == kHeatBlock ? 1 : H.form == kHeatCluster ? kHeatClusterSize
+                                                     : std::min((long)sm_count, (need + 255) / 256);
+        if (need > most * blocks || (H.form == kHeatCluster && dbg_forms >= 1) || (H.form == kHeatGrid && dbg_forms >= 2)) continue;
+        H.blocks = (unsigned)blocks;
+        H.threads = (unsigned)(((need + blocks - 1) / blocks + 31) / 32 * 32);
+        if (H.form == kHeatBlock) return;
+        HeatSweeps kern;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        int n = 0;
+        cudaError_t e = heat_config(H, kern, cfg, attr);
+        if (e == cudaSuccess)
+            e = H.form == kHeatCluster ? cudaOccupancyMaxActiveClusters(&n, kern, &cfg)
+                                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, (int)H.threads, 0);
+        if (e != cudaSuccess) cudaGetLastError();
+        else if (H.form == kHeatCluster ? n >= 1 : (long)n * sm_count >= blocks) return;
+    }
+}
+
 // The sweeps of a smoothing call, and the residual where the next kernel restricts it.
 void Solver::heat_smooth(int l, int sweeps, double t0koef, bool resid)
 {
-    const HeatLv V = heat_view(L[l], heat.lv[l], heat, l);
-    const HeatBc B = heat_bc_view(heat.lv[l]);
+    const HeatLevel &H = heat.lv[l];
+    const HeatLv V = heat_view(L[l], H, heat, l);
+    const HeatBc B = heat_bc_view(H);
     const long half = V.nh;
-    if (sweeps > 0) {
-        // one block while a thread per node of a colour and per boundary row fits, then a cluster (its barrier
-        // is the cheaper one), then a block per SM: each form is the fastest where it fits (k_heat_sweeps);
-        // a larger level's coefficients do not fit the registers, and it takes a launch per colour
-        const long need = std::max(half, (long)B.nbc), most = kHeatThreads;
-        const int form = need <= most ? kHeatBlock : need <= most * kHeatClusterSize ? kHeatCluster : kHeatGrid;
-        if (need <= most * sm_count) {
-            const long blocks = form == kHeatBlock ? 1 : form == kHeatCluster ? kHeatClusterSize
-                                                       : std::min((long)sm_count, (need + 255) / 256);
-            const GridBarrier S{heat.count, heat.scal + 7};
-            auto kern = form == kHeatBlock ? k_heat_sweeps<kHeatBlock>
-                        : form == kHeatCluster ? k_heat_sweeps<kHeatCluster> : k_heat_sweeps<kHeatGrid>;
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute attr[1];
-            cfg.gridDim = dim3((unsigned)blocks);
-            cfg.blockDim = dim3((unsigned)(((need + blocks - 1) / blocks + 31) / 32 * 32));
-            cfg.stream = st;
-            cfg.attrs = attr;
-            cfg.numAttrs = form != kHeatBlock;
-            if (form == kHeatCluster) {
-                // the same value from every thread: the attribute belongs to the function, not to this context
-                P2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-                attr[0].id = cudaLaunchAttributeClusterDimension;
-                attr[0].val.clusterDim.x = (unsigned)blocks;
-                attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-            } else {
-                attr[0].id = cudaLaunchAttributeCooperative;
-                attr[0].val.cooperative = 1;
-            }
-            P2_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, V, B, sweeps, t0koef, (int)(l == 0), (int)resid, S));
-            heat.kernels++;
-            return;
-        }
+    if (sweeps > 0 && H.form != kHeatPasses) {
+        HeatSweeps kern;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        P2_CUDA_TRY(heat_config(H, kern, cfg, attr));
+        cfg.stream = st;
+        const GridBarrier S{heat.count, heat.scal + 7};
+        P2_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, V, B, sweeps, t0koef, (int)(l == 0), (int)resid, S));
+        heat.kernels++;
+        return;
     }
     for (int s = 0; s < sweeps; s++)
         for (int c = 0; c < 2; c++) {

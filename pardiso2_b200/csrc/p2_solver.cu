@@ -623,22 +623,82 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
     bc_ready = true;
 }
 
-// Resident sweeps (p2_resident.cuh): whether the level's cells fit, in which
-// form, and the boundary rows that follow each cell's unknowns.
+// The launch of a level's resident sweeps in the form Lv.res_mode (1: one
+// cluster, 2: a cooperative grid).  The function attributes are the same from
+// every thread: they belong to the function, not to this context.
+template <typename T>
+using ResidentKernel = void (*)(LevelView<T>, Vec4<T>, Vec4<T>, Vec4<T>, T, int, const factor_t<T> *, long, ResidentBC, int,
+                                const T *, GridBarrier);
+template <typename T, bool kFull>
+static cudaError_t resident_config(const Level &Lv, ResidentKernel<T> &kern, cudaLaunchConfig_t &cfg,
+                                   cudaLaunchAttribute attr[2])
+{
+    const bool cluster = Lv.res_mode == 1;
+    kern = cluster ? k_smooth_resident<T, kFull, true> : k_smooth_resident<T, kFull, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemMax);
+    if (e == cudaSuccess && cluster) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cfg = {};
+    cfg.gridDim = dim3(Lv.res_blocks);
+    cfg.blockDim = dim3(2 * Lv.res_slots);
+    cfg.dynamicSmemBytes = res_smem<T, kFull>(2 * Lv.res_slots, Lv.tabstride, Lv.res_cap);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = Lv.res_blocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    }
+    return e;
+}
+
+// Whether the device can place that launch: the cluster's 16 blocks, or all
+// blocks of the grid at once.
+template <typename T, bool kFull>
+static bool resident_placed(const Level &Lv, int sm_count)
+{
+    ResidentKernel<T> kern;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    cudaError_t e = resident_config<T, kFull>(Lv, kern, cfg, attr);
+    if (e == cudaSuccess)
+        e = Lv.res_mode == 1 ? cudaOccupancyMaxActiveClusters(&n, kern, &cfg)
+                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, (int)cfg.blockDim.x, cfg.dynamicSmemBytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return Lv.res_mode == 1 ? n >= 1 : (long)n * sm_count >= Lv.res_blocks;
+}
+
+// Resident sweeps (p2_resident.cuh): one cluster where the level's cells fit and
+// the device places it, else a cooperative grid likewise, else passes of their
+// own.  The kernels of both smoothers have to be placed (the smoother can be
+// changed later).
 void Solver::build_resident(Level &Lv)
 {
-    const long half = Lv.ny / 2, slots = (long)(Lv.nx - 1) * (Lv.nz - 1) * half;
-    Lv.res_mode = 0;
-    auto per_block = [&](long blocks) { return (int)(((slots + blocks - 1) / blocks + 31) / 32 * 32); };
-    if (per_block(kResCluster) <= kResSlots) {
-        Lv.res_mode = 1;
-        Lv.res_blocks = kResCluster;
-    } else if (per_block(sm_count) <= kResSlots) {
-        Lv.res_mode = 2;
-        Lv.res_blocks = (int)((slots + per_block(sm_count) - 1) / per_block(sm_count));
-    } else {
-        return;
+    for (Lv.res_mode = 1 + std::min(dbg_forms, 2); Lv.res_mode <= 2; Lv.res_mode++) {
+        if (!build_resident_rows(Lv)) continue;
+        const bool placed = prm.precision == 0
+                                ? resident_placed<float, true>(Lv, sm_count) && resident_placed<float, false>(Lv, sm_count)
+                                : resident_placed<double, true>(Lv, sm_count) && resident_placed<double, false>(Lv, sm_count);
+        if (placed) return;
     }
+    Lv.res_mode = 0;
+}
+
+// The boundary rows that follow each cell's unknowns, for the form Lv.res_mode;
+// false where its blocks cannot hold the level.
+bool Solver::build_resident_rows(Level &Lv)
+{
+    const long half = Lv.ny / 2, slots = (long)(Lv.nx - 1) * (Lv.nz - 1) * half;
+    auto per_block = [&](long blocks) { return (int)(((slots + blocks - 1) / blocks + 31) / 32 * 32); };
+    const int most_blocks = Lv.res_mode == 1 ? kResCluster : sm_count;
+    if (per_block(most_blocks) > kResSlots) return false;
+    Lv.res_blocks = Lv.res_mode == 1 ? kResCluster : (int)((slots + per_block(sm_count) - 1) / per_block(sm_count));
     Lv.res_slots = per_block(Lv.res_blocks);
     // two passes over the rows: count per colour and slot, then place
     std::vector<int> ptr(2 * slots + 1, 0), at;
@@ -679,12 +739,10 @@ void Solver::build_resident(Level &Lv)
     Lv.res_cap = (Lv.res_cap + 1) / 2 * 2;
     const size_t most = std::max(res_smem<double, true>(2 * Lv.res_slots, Lv.tabstride, Lv.res_cap),
                                  res_smem<float, true>(2 * Lv.res_slots, Lv.tabstride, Lv.res_cap));
-    if (most > kResSmemMax) {
-        Lv.res_mode = 0;
-        return;
-    }
+    if (most > kResSmemMax) return false;
     Lv.res_ptr = upload(arena, ptr);
     Lv.res_dep = upload(arena, dep);
+    return true;
 }
 
 void Solver::allocate_work()
@@ -1256,33 +1314,18 @@ void Solver::smooth_resident(int l, int sweeps)
 {
     Level &Lv = L[l];
     LevelView<T> V = view<T>(l, false);
-    const int threads = 2 * Lv.res_slots, mx = Lv.tabstride;
-    const size_t smem = res_smem<T, kFull>(threads, mx, Lv.res_cap);
+    const int mx = Lv.tabstride;
     const ResidentBC R{Lv.nbc, Lv.bu, Lv.bt, Lv.bnext, Lv.bk, Lv.res_ptr, Lv.res_dep, Lv.res_cap};
     const T *tab = std::is_same<T, double>::value ? (const T *)Lv.tabd : (const T *)Lv.tabf;
-    const bool cluster = Lv.res_mode == 1;
-    auto kern = cluster ? k_smooth_resident<T, kFull, true> : k_smooth_resident<T, kFull, false>;
-    // the same value from every thread: the attribute belongs to the function, not to this context
-    P2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemMax));
-    if (cluster) P2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(Lv.res_blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
+    ResidentKernel<T> kern;
+    cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    cfg.attrs = attr;
-    if (cluster) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = Lv.res_blocks;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    P2_CUDA_TRY((resident_config<T, kFull>(Lv, kern, cfg, attr)));
+    cfg.stream = st;
+    if (Lv.res_mode == 1) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
-    } else {
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.numAttrs = 1;
     }
     P2_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, V, vx_of<T>(Lv, 0), vx_of<T>(Lv, 1), b_of<T>(Lv), (T)prm.omega, 2 * sweeps,
                                    (const factor_t<T> *)Lv.blk, Lv.blk_stride, R, mx, tab,

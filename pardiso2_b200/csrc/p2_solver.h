@@ -90,6 +90,8 @@ struct HeatLevel {
     float *kt = nullptr, *cp = nullptr, *ro = nullptr;  // coarse levels (level 0: HeatState)
     double *x = nullptr, *b = nullptr, *r = nullptr, *a = nullptr;  // b, a in colour order
     long nh = 0;                          // nodes per colour slot range
+    int form = 0;                         // of its sweeps (k_heat_sweeps), and that launch
+    unsigned blocks = 0, threads = 0;
     AxisMap map[3]{};                     // this level -> next coarser level
 };
 
@@ -165,6 +167,7 @@ class Solver {
     double debug_time_sweep(int level, int sweeps);
     double debug_time_stage(int stage, int level, int variant, int reps);
     int dbg_rows_variant = 0;     // kernel of the operator rows (launch_rows), 0 = by grid size and precision
+    int dbg_forms = 0;            // resident sweeps as if the device placed no cluster (1), nor a cooperative grid (2)
     void drop_graphs_public() { drop_graphs(); }
     void debug_smooth(int level, int sweeps, const double *b, double *x);
     void debug_vcycle(const double *b, double *x);
@@ -227,6 +230,7 @@ class Solver {
     template <typename T, bool kFull>
     void smooth_resident(int l, int sweeps);
     void build_resident(Level &Lv);
+    bool build_resident_rows(Level &Lv);
     int sm_count = 0;
     unsigned *res_count = nullptr;  // grid barrier counters of the resident sweeps
     template <typename T>
@@ -260,6 +264,7 @@ class Solver {
     void reserve_move_positions(long nmark);
     void velocity_f32();
 
+    void heat_choose_form(HeatLevel &H);
     void heat_smooth(int l, int sweeps, double t0koef, bool resid);
     void heat_batch(const p2_heat_params &hp);
 
