@@ -162,16 +162,23 @@ __device__ __forceinline__ void gj_invert(const double *sh, double *w, double *D
     }
 }
 
+// +-1 by the bits of a hash of r
+__device__ __forceinline__ double gj_sign(int r)
+{
+    unsigned h = (unsigned)r * 2654435761u;
+    h ^= h >> 15;
+    return (h & 0x400u) ? 1.0 : -1.0;
+}
+
 // X = A in the permuted order with identity padding, column-major n x n; the
-// columns along the grid's x, whose y ends at 65535
-__global__ void k_gj_gather(int n, int nF, const int *perm, const double *A, double *X)
+// columns along the grid's x, whose y ends at 65535.  v: the check's vector.
+__global__ void k_gj_gather(int n, int nF, const int *perm, const double *A, const double *scale, double *X, double *v)
 {
     const int r = blockIdx.y * blockDim.x + threadIdx.x, c = blockIdx.x;
     if (r >= n) return;
     const int pr = perm[r], pc = perm[c];
-    double v = r == c ? 1.0 : 0.0;
-    if (pr >= 0 && pc >= 0) v = A[(size_t)pc * nF + pr];
-    X[(size_t)c * n + r] = v;
+    if (r == 0) v[c] = pc >= 0 ? gj_sign(c) * scale[pc] : 0.0;
+    X[(size_t)c * n + r] = pr >= 0 && pc >= 0 ? A[(size_t)pc * nF + pr] : (r == c ? 1.0 : 0.0);
 }
 
 __global__ void __launch_bounds__(kGThreads) k_gj_first(const double *X, int n, double *D, int *flag)
@@ -300,16 +307,15 @@ __global__ void __launch_bounds__(kGThreads, 3) k_gj_update(double *X, int n, in
     }
 }
 
-// Check of the inverse: y = X v for v_r = +-1 by the bits of a hash of r, then
-// flag when a row of A y - v is above kGjCheck (or not a number).
+// Check of the inverse: y = X v for v_r = +-s_r with the rows' scales s_r (their
+// largest velocity entries), then flag when |A y - v| in a row is above kGjCheck
+// s_r (or not a number).  That is the test of the inverse of A with its rows
+// scaled to 1, so it does not depend on the units: rounding alone leaves about
+// 1e-14 at equal viscosities and 1e-7 at a contrast of 1e4, in a unit box as in
+// metres and Pa s, where an absolute bound on v = +-1 fails any inverse
+// (momentum rows hold eta / h^2, continuity rows 1 / h).
 constexpr double kGjCheck = 1e-4;
-__device__ __forceinline__ double gj_sign(int r)
-{
-    unsigned h = (unsigned)r * 2654435761u;
-    h ^= h >> 15;
-    return (h & 0x400u) ? 1.0 : -1.0;
-}
-// row r of A b (b null: the signs), the 32 warps of the block splitting the columns
+// row r of A b, the 32 warps of the block splitting the columns
 constexpr int kCheckWarps = 32;
 __device__ __forceinline__ double gj_rows(int n, const double *A, int r, const double *b, double (*part)[33])
 {
@@ -317,7 +323,7 @@ __device__ __forceinline__ double gj_rows(int n, const double *A, int r, const d
     double s = 0;
     if (r < n) {
 #pragma unroll 4
-        for (int c = w; c < n; c += kCheckWarps) s += A[(size_t)c * n + r] * (b ? b[c] : gj_sign(c));
+        for (int c = w; c < n; c += kCheckWarps) s += A[(size_t)c * n + r] * b[c];
     }
     part[w][lane] = s;
     __syncthreads();
@@ -325,20 +331,24 @@ __device__ __forceinline__ double gj_rows(int n, const double *A, int r, const d
     for (int q = 0; q < kCheckWarps; q++) t += part[q][lane];
     return t;
 }
-__global__ void __launch_bounds__(32 * kCheckWarps) k_gj_check_x(int n, const int *perm, const double *X, double *y)
+__global__ void __launch_bounds__(32 * kCheckWarps) k_gj_check_x(int n, const int *perm, const double *X, const double *v,
+                                                                 double *y)
 {
     __shared__ double part[kCheckWarps][33];
     const int r = blockIdx.x * 32 + (threadIdx.x & 31);
-    const double t = gj_rows(n, X, r, nullptr, part);
+    const double t = gj_rows(n, X, r, v, part);
     if (threadIdx.x < 32 && r < n && perm[r] >= 0) y[perm[r]] = t;  // y in the order of A
 }
 __global__ void __launch_bounds__(32 * kCheckWarps) k_gj_check_a(int nF, const int *iperm, const double *A,
-                                                                 const double *y, int *flag)
+                                                                 const double *y, const double *v, int *flag)
 {
     __shared__ double part[kCheckWarps][33];
     const int r = blockIdx.x * 32 + (threadIdx.x & 31);
     const double t = gj_rows(nF, A, r, y, part);
-    if (threadIdx.x < 32 && r < nF && !(fabs(t - gj_sign(iperm[r])) < kGjCheck)) *flag = 2;
+    if (threadIdx.x < 32 && r < nF) {
+        const double want = v[iperm[r]];
+        if (!(fabs(t - want) < kGjCheck * fabs(want))) *flag = 2;
+    }
 }
 
 }  // namespace p2

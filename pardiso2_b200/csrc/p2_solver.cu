@@ -52,7 +52,7 @@ constexpr double kOverlapScale = 60.0;
 constexpr int kOverlapMax = 16;
 void d2f(cudaStream_t st, size_t n, const double *a, float *b);
 size_t gj_work_doubles(int n);
-void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
+void gj_inverse(cudaStream_t st, const double *A, const double *scale, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
                 LuGraph *cache);
 void permute_inverse(cudaStream_t st, const GjPlan &P, const double *B, double *X);
 
@@ -943,6 +943,7 @@ void Solver::build_coarse_index()
     Ainv64 = (double *)arena.alloc(sizeof(double) * (size_t)gj.n * gj.n);
     Ainv32 = (float *)arena.alloc(sizeof(float) * (size_t)gj.n * gj.n);
     gj_work = (double *)arena.alloc(sizeof(double) * gj_work_doubles(gj.n));
+    d_row_scale = (double *)arena.alloc(sizeof(double) * nF);
     d_ipiv = (int *)arena.alloc(sizeof(int) * nF);
     d_info = (int *)arena.alloc(sizeof(int) * 4);
     probes = (double *)arena.alloc(sizeof(double) * (size_t)C.n * 4 * kProbes);
@@ -965,7 +966,7 @@ void Solver::build_coarse_index()
 // within two nodes.  All kProbes probes are built and applied in one launch
 // each (blockIdx.y = probe); the row kernel also records the band of the
 // operator in the free-unknown ordering (bw[0] = max row - col, bw[1] = max
-// col - row over the non-zeros).
+// col - row over the non-zeros) and every row's scale, its largest velocity entry.
 
 __global__ void k_probe_build(int nx, int ny, int nz, const int *colmap, const int *rt, const float *rk,
                               double *probes)
@@ -992,7 +993,7 @@ __global__ void k_probe_build(int nx, int ny, int nz, const int *colmap, const i
 }
 
 __global__ void k_probe_rows(LevelView<double> Lc, const double *probes, const int *colmap, double *A, int nF,
-                             int *bw)
+                             int *bw, unsigned long long *scale)
 {
     int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= Lc.n) return;
@@ -1022,6 +1023,7 @@ __global__ void k_probe_rows(LevelView<double> Lc, const double *probes, const i
         if (a != 0.0) {
             if (row > col) atomicMax(&bw[0], row - col);
             if (col > row) atomicMax(&bw[1], col - row);
+            if (comp) atomicMax(scale + row, (unsigned long long)__double_as_longlong(fabs(a)));  // orders as the values do
         }
     }
 }
@@ -1039,7 +1041,8 @@ void Solver::coarse_setup(int way)
     P2_CUDA_TRY(cudaMemsetAsync(d_bw, 0, sizeof(int) * 2, st));
     dim3 grid(nblk(C.n), kProbes);
     k_probe_build<<<grid, kThreads, 0, st>>>(C.nx, C.ny, C.nz, d_colmap, d_crt, d_crk, probes); P2_COUNT_LAUNCH();
-    k_probe_rows<<<grid, kThreads, 0, st>>>(Lc, probes, d_colmap, A_c, nF, d_bw); P2_COUNT_LAUNCH();
+    P2_CUDA_TRY(cudaMemsetAsync(d_row_scale, 0, sizeof(double) * nF, st));
+    k_probe_rows<<<grid, kThreads, 0, st>>>(Lc, probes, d_colmap, A_c, nF, d_bw, (unsigned long long *)d_row_scale); P2_COUNT_LAUNCH();
     P2_CUDA_TRY(cudaGetLastError());
     // The inverse runs on its own stream; the solve goes on with a smoothed
     // coarsest level for lu_overlap_iters outer iterations.
@@ -1049,7 +1052,7 @@ void Solver::coarse_setup(int way)
     if (lu_pivoted) {
         invert_pivoted();
     } else {
-        gj_inverse(st_lu, A_c, gj, Ainv64, prm.precision == 0 ? Ainv32 : nullptr, gj_work, d_info, &lu_graph);
+        gj_inverse(st_lu, A_c, d_row_scale, gj, Ainv64, prm.precision == 0 ? Ainv32 : nullptr, gj_work, d_info, &lu_graph);
         P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
     }
     lu_pending = true;

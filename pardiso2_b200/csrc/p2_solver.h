@@ -304,7 +304,7 @@ class Solver {
     int *d_colmap = nullptr, *d_crt = nullptr;
     GjPlan gj;
     int *d_slots = nullptr, *d_slot_of = nullptr;  // unknown of each slot of the inverse (-1 padding), and back
-    double *gj_work = nullptr;
+    double *gj_work = nullptr, *d_row_scale = nullptr;
     LuGraph lu_graph_pivoted;
     void invert_pivoted();
     bool lu_pivoted = false;  // the inverse in flight is the pivoted LU's
