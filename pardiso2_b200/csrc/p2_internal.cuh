@@ -398,9 +398,11 @@ struct TransferView {
     AxisMap m[3][3];  // [axis][type]
 };
 
+// Boundary rows that follow a regular unknown: row, resolved target and the
+// product of the chain's coefficients in the cycle's type.
 struct BcFollow {
     int n;
     const int *uc, *target;
-    const float *k;
+    const void *k;
 };
 }  // namespace p2

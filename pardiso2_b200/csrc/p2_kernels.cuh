@@ -196,7 +196,7 @@ __global__ void k_bc_follow(BcFollow R, const T *c, Vec4<T> x)
     const int uc = __ldg(R.uc + q), t = __ldg(R.target + q);
     const T *s = (t & 3) == 0 ? x.c[0] : ((t & 3) == 1 ? x.c[1] : ((t & 3) == 2 ? x.c[2] : x.c[3]));
     T *d = (uc & 3) == 0 ? x.c[0] : ((uc & 3) == 1 ? x.c[1] : ((uc & 3) == 2 ? x.c[2] : x.c[3]));
-    d[uc >> 2] = __ldg(c + q) + (T)__ldg(R.k + q) * s[t >> 2];
+    d[uc >> 2] = __ldg(c + q) + __ldg((const T *)R.k + q) * s[t >> 2];
 }
 // Start of a smoothing call: every boundary row of x (as k_bc_set_chain) and,
 // in the second velocity buffer y, the same values, which the rows without a

@@ -30,14 +30,15 @@ constexpr int kResCluster = 16;
 
 // Boundary rows for the resident sweeps: the rows' chains as for
 // k_bc_set_chain, and per colour and slot the rows that follow one of the
-// cell's unknowns: {face 0..5 or 6 for the pressure, unknown, row, product of
-// the chain's coefficients as bits}.
+// cell's unknowns: {unknown * 8 + face (0..5, 6 for the pressure), row} and the
+// product of the chain's coefficients in the cycle's type.
 struct ResidentBC {
     int nbc;
     const int *bu, *bt, *bnext;
     const float *bk;
     const int *ptr;
-    const int4 *dep;
+    const int2 *dep;
+    const void *depk;
     int cap;  // most entries of one block
 };
 
@@ -58,8 +59,7 @@ __host__ __device__ constexpr int res_values() { return kFull ? kBlkEntries : 7;
 // a row that follows an unknown of the block's cells: its constant part, coefficient, unknown and face
 template <typename T>
 struct ResDep {
-    T c;
-    float k;
+    T c, k;
     int what;  // unknown * 8 + face
 };
 constexpr size_t kResSmemMax = 227 * 1024 - 64;
@@ -160,8 +160,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_smooth_resident(LevelView<T>
         y.c[uc & 3][uc >> 2] = v;
     }
     for (int e = tid; e < n0 + n1; e += nt) {
-        const int4 D = R.dep[e < n0 ? e0 + e : e1 + e - n0];
-        deps[e] = ResDep<T>{row_value(D.z, true), __int_as_float(D.w), D.y * 8 + D.x};
+        const int at = e < n0 ? e0 + e : e1 + e - n0;
+        const int2 D = R.dep[at];
+        deps[e] = ResDep<T>{row_value(D.y, true), ((const T *)R.depk)[at], D.x};
     }
     __syncthreads();  // the tables and entries
     if (!kFull && valid) {
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_smooth_resident(LevelView<T>
                 const T v = face == 0 ? vn[0] : face == 1 ? vn[1] : face == 2 ? vn[2] : face == 3 ? vn[3]
                           : face == 4 ? vn[4] : face == 5 ? vn[5] : p;
                 T *o = (uc & 3) == 0 ? o0 : ((uc & 3) == 1 ? o1 : ((uc & 3) == 2 ? o2 : o3));
-                o[uc >> 2] = D.c + (T)D.k * v;
+                o[uc >> 2] = D.c + D.k * v;
             }
         }
         swap(i0, o0); swap(i1, o1); swap(i2, o2); swap(i3, o3);

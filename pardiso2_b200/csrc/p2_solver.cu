@@ -15,7 +15,6 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
-#include <cstring>
 #include <map>
 #include <memory>
 #include <string>
@@ -216,6 +215,13 @@ static V *upload(DeviceArena &A, const std::vector<V> &h)
     V *d = (V *)A.alloc(sizeof(V) * std::max<size_t>(h.size(), 1));
     if (!h.empty()) P2_CUDA_TRY(cudaMemcpy(d, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice));
     return d;
+}
+
+// Values in the V-cycle's type.
+void *Solver::upload_cycle(const std::vector<double> &v)
+{
+    if (prm.precision == 1) return upload(arena, v);
+    return upload(arena, std::vector<float>(v.begin(), v.end()));
 }
 
 static AxisMap upload_axis(DeviceArena &A, const HostAxis &h, bool restriction = false)
@@ -599,15 +605,15 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
         build_resident(Lv);
         if (!Lv.res_mode) {
             std::vector<int> slot(Lv.h_bu.size(), -1), uc, target;
-            std::vector<float> k;
+            std::vector<double> k;
             for (size_t q = 0; q < Lv.h_bu.size(); q++) {
                 if (Lv.h_rt[q] < 0) continue;
                 slot[q] = (int)uc.size();
                 uc.push_back(Lv.h_bu[q]);
                 target.push_back(Lv.h_rt[q]);
-                k.push_back((float)Lv.h_rk[q]);
+                k.push_back(Lv.h_rk[q]);
             }
-            Lv.follow = BcFollow{(int)uc.size(), upload(arena, uc), upload(arena, target), upload(arena, k)};
+            Lv.follow = BcFollow{(int)uc.size(), upload(arena, uc), upload(arena, target), upload_cycle(k)};
             Lv.follow_slot = upload(arena, slot);
             Lv.follow_const = arena.alloc(sizeof(double) * std::max<size_t>(uc.size(), 1));
         }
@@ -702,22 +708,24 @@ bool Solver::build_resident_rows(Level &Lv)
     Lv.res_slots = per_block(Lv.res_blocks);
     // two passes over the rows: count per colour and slot, then place
     std::vector<int> ptr(2 * slots + 1, 0), at;
-    std::vector<int4> dep;
+    std::vector<int2> dep;
+    std::vector<double> depk;
     for (int pass = 0; pass < 2; pass++) {
         for (size_t q = 0; q < Lv.h_bu.size(); q++) {
             const int t = Lv.h_rt[q];
             if (t < 0) continue;
-            const float rk = (float)Lv.h_rk[q];
             const int c = t & 3, v = t >> 2;
             const int j = v % Lv.ny, i = (v / Lv.ny) % Lv.nx, k = v / (Lv.nx * Lv.ny);
-            int kbits;
-            std::memcpy(&kbits, &rk, sizeof kbits);
             auto follow = [&](int ci, int cj, int ck, int face) {
                 // a target that is no cell's unknown keeps its value through the sweeps
                 if (ci < 1 || cj < 1 || ck < 1 || ci >= Lv.nx || cj >= Lv.ny || ck >= Lv.nz) return;
                 const long slot = ((ci + cj + ck) & 1) * slots + ((long)(ck - 1) * (Lv.nx - 1) + (ci - 1)) * half + (cj - 1) / 2;
-                if (pass == 0) ptr[slot + 1]++;
-                else dep[at[slot]++] = make_int4(face, Lv.h_bu[q], (int)q, kbits);
+                if (pass == 0) {
+                    ptr[slot + 1]++;
+                } else {
+                    depk[at[slot]] = Lv.h_rk[q];
+                    dep[at[slot]++] = make_int2(Lv.h_bu[q] * 8 + face, (int)q);
+                }
             };
             // the cells on both sides of a face (one of each colour), or the pressure's own cell
             if (c == 0) follow(i, j, k, 6);
@@ -729,6 +737,7 @@ bool Solver::build_resident_rows(Level &Lv)
             for (long e = 0; e < 2 * slots; e++) ptr[e + 1] += ptr[e];
             at.assign(ptr.begin(), ptr.end() - 1);
             dep.resize(ptr[2 * slots]);
+            depk.resize(ptr[2 * slots]);
         }
     }
     Lv.res_cap = 0;
@@ -742,6 +751,7 @@ bool Solver::build_resident_rows(Level &Lv)
     if (most > kResSmemMax) return false;
     Lv.res_ptr = upload(arena, ptr);
     Lv.res_dep = upload(arena, dep);
+    Lv.res_depk = upload_cycle(depk);
     return true;
 }
 
@@ -1318,7 +1328,7 @@ void Solver::smooth_resident(int l, int sweeps)
     Level &Lv = L[l];
     LevelView<T> V = view<T>(l, false);
     const int mx = Lv.tabstride;
-    const ResidentBC R{Lv.nbc, Lv.bu, Lv.bt, Lv.bnext, Lv.bk, Lv.res_ptr, Lv.res_dep, Lv.res_cap};
+    const ResidentBC R{Lv.nbc, Lv.bu, Lv.bt, Lv.bnext, Lv.bk, Lv.res_ptr, Lv.res_dep, Lv.res_depk, Lv.res_cap};
     const T *tab = std::is_same<T, double>::value ? (const T *)Lv.tabd : (const T *)Lv.tabf;
     ResidentKernel<T> kern;
     cudaLaunchConfig_t cfg;

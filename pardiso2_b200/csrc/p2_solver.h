@@ -53,7 +53,8 @@ struct Level {
     // resident sweeps (k_smooth_resident): 0 none, 1 one cluster, 2 cooperative grid
     int res_mode = 0, res_blocks = 0, res_slots = 0, res_cap = 0;
     int *res_ptr = nullptr;
-    int4 *res_dep = nullptr;
+    int2 *res_dep = nullptr;
+    void *res_depk = nullptr;
     // boundary rows between separate colour passes
     BcFollow follow{};
     int *follow_slot = nullptr;
@@ -229,6 +230,7 @@ class Solver {
     void smooth(int l, int sweeps);
     template <typename T, bool kFull>
     void smooth_resident(int l, int sweeps);
+    void *upload_cycle(const std::vector<double> &v);
     void build_resident(Level &Lv);
     bool build_resident_rows(Level &Lv);
     int sm_count = 0;
