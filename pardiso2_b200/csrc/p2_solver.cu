@@ -2162,8 +2162,7 @@ double Solver::debug_time_stage(int stage, int l, int variant, int reps)
                 if (f32) level_residual<float>(l);
                 else level_residual<double>(l);
             } else if (stage == 1) {
-                // the float copy goes where solve() puts it: the restriction relies on r32 being 0 on boundary rows
-                rows0(gx, gr, f32 ? &L[0].b32 : nullptr, 0);
+                rows0(gx, gr, f32 ? &L[0].r32 : nullptr, 0);
             } else if (stage == 4) {
                 if (f32) rows0(Z32[0], W[1], nullptr, 1);
                 else rows0(Z64[0], W[1], nullptr, 1);
