@@ -1598,6 +1598,7 @@ p2_solve_info Solver::solve()
     // iteration with k stored ones where GCR moved 5 k + 12 and the residual rows.
     // At 257^3 the outer loop went from 6.27 to 3.54 ms per iteration (V-cycle 12.8).
     std::vector<double> R((size_t)m * m), cs(m), sn(m), g(m + 1), nrm(m + 1), y(m);
+    bool bad = false;  // a direction without a positive norm, or not a number
     for (;;) {
         // true FP64 residual, with its copy for the V-cycle
         rows0(gx, W[0], f32 ? &L0.b32 : nullptr, 0);
@@ -1608,10 +1609,10 @@ p2_solve_info Solver::solve()
         if (verbose) std::fprintf(stderr, "p2cuda: iteration %d rel residual %.3e\n", it, rel);
         if (!std::isfinite(rel)) { info.status = P2_ERR_NAN; break; }
         if (rel <= prm.tol) { info.status = P2_OK; break; }
+        if (bad) { info.status = P2_ERR_NAN; break; }
         if (it >= prm.max_iter) { info.status = P2_ERR_NOT_CONVERGED; break; }
         nrm[0] = g[0] = std::sqrt(rr);
         int k = 0;
-        bool bad = false;
         while (k < m && it < prm.max_iter) {
             if (it >= lu_overlap_iters) lu_finish();
             coarse_mode = lu_pending ? 1 : 0;
@@ -1652,7 +1653,6 @@ p2_solve_info Solver::solve()
                 throw Error(P2_ERR_CUDA, "a grid barrier of the smoother ran out of time");
             }
             const double sigma = hc[HC_SIGMA], wn2 = hc[HC_WW];
-            // a direction without a positive norm, or not a number
             if (!(hc[HC_QQ] > 0) || !std::isfinite(wn2) || !std::isfinite(hc[HC_QQ])) { bad = true; break; }
             nrm[k + 1] = std::sqrt(wn2);
             double *col = &R[(size_t)k * m];
@@ -1664,6 +1664,7 @@ p2_solve_info Solver::solve()
                 col[j] = t;
             }
             const double d = std::hypot(col[k], sub);
+            if (!(d > 0) || !std::isfinite(d)) { bad = true; break; }
             cs[k] = col[k] / d;
             sn[k] = sub / d;
             col[k] = d;
@@ -1674,8 +1675,7 @@ p2_solve_info Solver::solve()
             if (verbose) std::fprintf(stderr, "p2cuda: iteration %d rel residual %.3e (estimate)\n", it, rel);
             if (rel <= prm.tol || !(wn2 > 0)) break;
         }
-        if (bad) { info.status = P2_ERR_NAN; break; }
-        // x += sum y_j Z_j, y = R^-1 g
+        // x += sum y_j Z_j, y = R^-1 g; the directions before a bad one count
         for (int i = k - 1; i >= 0; i--) {
             double s = g[i];
             for (int j = i + 1; j < k; j++) s -= R[(size_t)j * m + i] * y[j];
