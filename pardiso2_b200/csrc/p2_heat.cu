@@ -869,7 +869,7 @@ void Solver::heat_set_bc(const int *bondm, long bondm_len, const float *bondv1, 
         heat.mev = e2;
     }
     heat.stage = std::make_shared<HostStage>();
-    heat.stage->reserve();
+    if (n0 >= HostStage::kLikelyNodes) heat.stage->reserve();
     P2_CUDA_TRY(cudaMallocHost((void **)&heat.host, sizeof(double) * 8));  // [0..3] error, range; [4] sub-step; [6] marker range; [7] barrier
     heat.host_owner.reset(heat.host, [](double *p) { cudaFreeHost(p); });
     P2_CUDA_TRY(cudaStreamSynchronize(st));

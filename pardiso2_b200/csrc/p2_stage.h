@@ -31,6 +31,14 @@ class HostStage {
   public:
     static constexpr size_t kPiece = (size_t)256 << 10;
     static constexpr int kWorkers = 4, kSlots = 3;
+    // The slots are made (3 to 4 ms of page-locking) with the heat rows of a grid of
+    // at least kLikelyNodes nodes, on a smaller one when a list of at least kLeast
+    // pageable bytes arrives; from then on every list goes through them.  Heat steps
+    // with / without: fields and markers of 3 + 4 MB 5.56 / 5.52 ms, 6 + 9 MB 5.84 /
+    // 5.88, 10 + 15 MB 5.76 / 6.10, 23 + 4 MB 5.39 / 5.92, 23 + 36 MB 6.9 / 9.4: a small
+    // step would not earn them.
+    static constexpr long kLikelyNodes = 50000;
+    static constexpr size_t kLeast = 40 * kPiece;
 
     ~HostStage()
     {
@@ -41,27 +49,47 @@ class HostStage {
             }
         if (buf) cudaFreeHost(buf);
     }
-    void reserve()
+    // The slots and their events; false when the host gives no page-locked memory.
+    bool reserve()
     {
-        if (buf) return;
+        if (buf) return true;
         const unsigned hw = std::thread::hardware_concurrency();
         workers = (int)std::min<unsigned>(kWorkers, std::max(1u, hw / 2));
-        ev.assign((size_t)workers * kSlots, nullptr);
-        for (cudaEvent_t &e : ev) P2_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        P2_CUDA_TRY(cudaMallocHost((void **)&buf, kPiece * workers * kSlots));
+        ev.resize((size_t)workers * kSlots, nullptr);
+        for (cudaEvent_t &e : ev)
+            if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+                e = nullptr;
+                cudaGetLastError();
+                return false;
+            }
+        if (cudaMallocHost((void **)&buf, kPiece * workers * kSlots) != cudaSuccess) {
+            buf = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+        return true;
     }
+
     // Issues the copies on the stream: page-locked arrays directly, others in
-    // pieces.  To the device: returns once the pageable arrays have been read.
-    // To the host: once they have been written.
+    // pieces (directly while there are no slots).  To the device: returns once the pageable
+    // arrays have been read.  To the host: once they have been written.
     cudaError_t run(int device, std::vector<HostCopy> list, cudaMemcpyKind kind, cudaStream_t st)
     {
         const bool up = kind == cudaMemcpyHostToDevice;
         struct Piece { char *dev, *host; size_t bytes; };
         std::vector<Piece> pieces;
-        for (const HostCopy &c : list) {
+        size_t total = 0;
+        std::vector<char> pageable(list.size());
+        for (size_t q = 0; q < list.size(); q++) {
             cudaPointerAttributes at{};
-            if (cudaPointerGetAttributes(&at, c.host) != cudaSuccess) cudaGetLastError();
-            if (at.type == cudaMemoryTypeHost || at.type == cudaMemoryTypeManaged || at.type == cudaMemoryTypeDevice) {
+            if (cudaPointerGetAttributes(&at, list[q].host) != cudaSuccess) cudaGetLastError();
+            pageable[q] = !(at.type == cudaMemoryTypeHost || at.type == cudaMemoryTypeManaged || at.type == cudaMemoryTypeDevice);
+            if (pageable[q]) total += list[q].bytes;
+        }
+        const bool staged = buf || (total >= kLeast && reserve());
+        for (size_t q = 0; q < list.size(); q++) {
+            const HostCopy &c = list[q];
+            if (!pageable[q] || !staged) {
                 const cudaError_t e = up ? cudaMemcpyAsync(c.dev, c.host, c.bytes, kind, st)
                                          : cudaMemcpyAsync(c.host, c.dev, c.bytes, kind, st);
                 if (e != cudaSuccess) return e;
@@ -70,6 +98,7 @@ class HostStage {
             for (size_t o = 0; o < c.bytes; o += kPiece)
                 pieces.push_back(Piece{(char *)c.dev + o, (char *)c.host + o, std::min(kPiece, c.bytes - o)});
         }
+        if (pieces.empty()) return cudaSuccess;
         std::atomic<size_t> next{0};
         std::atomic<int> error{(int)cudaSuccess};
         auto work = [&](int w) {
