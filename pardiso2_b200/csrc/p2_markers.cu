@@ -282,19 +282,21 @@ __global__ void k_cell_order(const unsigned *key, const unsigned *slot, long nma
 
 // start (the scanned counts) and end from the counts in end, idx and sorted from
 // key and pos; tot: per-block totals of the scan.
-static void launch_cell_sort(cudaStream_t st, long nmark, const unsigned *key, const unsigned *pos, unsigned sentinel,
-                             int *start, int *end, long ncell, unsigned *tot, unsigned *slot, const float *mx,
-                             const float *my, const float *mz, const signed char *mt, unsigned *idx, float4 *sorted,
-                             long long *launches)
+static cudaError_t launch_cell_sort(cudaStream_t st, long nmark, const unsigned *key, const unsigned *pos,
+                                    unsigned sentinel, int *start, int *end, long ncell, unsigned *tot, unsigned *slot,
+                                    const float *mx, const float *my, const float *mz, const signed char *mt, unsigned *idx,
+                                    float4 *sorted, long long *launches)
 {
     const unsigned sblocks = (unsigned)((ncell + kScanChunk - 1) / kScanChunk);
-    cudaMemcpyAsync(start, end, sizeof(int) * ncell, cudaMemcpyDeviceToDevice, st);
+    const cudaError_t e = cudaMemcpyAsync(start, end, sizeof(int) * ncell, cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return e;
     k_scan_local<<<sblocks, kScanThreads, 0, st>>>((unsigned *)start, ncell, tot);
     k_radix_scan<<<1, 1024, 0, st>>>(tot, (long)sblocks);
     k_cell_ranges<<<sblocks, kScanThreads, 0, st>>>(start, end, ncell, tot);
     k_cell_scatter<<<nb(nmark), 256, 0, st>>>(nmark, key, pos, sentinel, start, slot);
     k_cell_order<<<nb(nmark), 256, 0, st>>>(key, slot, nmark, start, end, ncell, mx, my, mz, mt, idx, sorted);
     *launches += 5;
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -1042,8 +1044,8 @@ void Solver::ronurecalc_device()
         P2_CUDA_TRY(cudaStreamSynchronize(st));
     }
     if (n > 0 && most == 0) {
-        launch_cell_sort(st, n, mk_key[0], mk_key[1], sentinel, cell_start, cell_end, ncell, mk_scan, mk_val[0], mk_x, mk_y,
-                         mk_z, mk_t, mk_val[1], mk_sorted, &g_launches);
+        P2_CUDA_TRY(launch_cell_sort(st, n, mk_key[0], mk_key[1], sentinel, cell_start, cell_end, ncell, mk_scan, mk_val[0],
+                                     mk_x, mk_y, mk_z, mk_t, mk_val[1], mk_sorted, &g_launches));
         mk_cur = 1;
     } else if (n > 0) {
         P2_CUDA_TRY(cudaMemsetAsync(cell_end, 0, sizeof(int) * ncell, st));
@@ -1279,8 +1281,8 @@ extern "C" p2_status p2_ronurecalc_noalloc(int nx, int ny, int nz, const double 
             return fail(err, errlen, P2_ERR_ARG, "%u markers have a type below 50 without a rock entry", seen[0]);
         if (seen[1] == 0) {
             long long launches = 0;
-            p2::launch_cell_sort(s, nmark, key[0], key[1], sentinel, cstart, cend, ncell, hist, val[0], markx, marky, markz,
-                                 markt, val[1], sorted, &launches);
+            P2NA_TRY(p2::launch_cell_sort(s, nmark, key[0], key[1], sentinel, cstart, cend, ncell, hist, val[0], markx,
+                                          marky, markz, markt, val[1], sorted, &launches));
             cur = 1;
             passes = -1;
         } else {
