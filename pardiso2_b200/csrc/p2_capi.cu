@@ -205,17 +205,19 @@ p2_status p2_stokes_solve_batch(p2_ctx *const *ctxs, int count, int host_threads
         P2_CUDA_TRY(cudaEventSynchronize(e0));
     });
     if (st0 == P2_OK) {
-        std::atomic<int> next{0};
-        auto work = [&] {
-            for (int q = next++; q < count; q = next++) {
-                const int i = order[q];
-                sts[i] = p2_stokes_solve_resident(ctxs[i], &res[i]);
-            }
-        };
         int nt = host_threads > 0 ? host_threads : count;
         const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
         if (host_threads <= 0) nt = std::min(nt, hw);
         nt = std::max(1, std::min(nt, count));
+        std::atomic<int> next{0};
+        auto work = [&] {
+            for (int q = next++; q < count; q = next++) {
+                const int i = order[q];
+                ctxs[i]->s->in_batch = nt > 1;
+                sts[i] = p2_stokes_solve_resident(ctxs[i], &res[i]);
+                ctxs[i]->s->in_batch = false;
+            }
+        };
         std::vector<std::thread> pool;
         try {
             for (int t = 1; t < nt; t++) pool.emplace_back(work);

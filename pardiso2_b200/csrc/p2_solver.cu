@@ -603,7 +603,7 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
             Lv.sw_order = upload(arena, order);
         }
         build_resident(Lv);
-        if (!Lv.res_mode) {
+        if (!Lv.res_mode || (Lv.res_mode == 2 && prm.precision == 0)) {
             std::vector<int> slot(Lv.h_bu.size(), -1), uc, target;
             std::vector<double> k;
             for (size_t q = 0; q < Lv.h_bu.size(); q++) {
@@ -1346,18 +1346,30 @@ void Solver::smooth_resident(int l, int sweeps)
     P2_COUNT_LAUNCH();
 }
 
+// The cooperative form keeps every SM for its launch, so among concurrent solves
+// the FP32 sweeps of the full cell block take a launch per pass on its levels, bit
+// for bit the same (a solve alone is 0 to 3 % faster with the grid): eight models of
+// 33^3 to 81^3 53.1 -> 50.4 ms, four of 49^3 to 97^3 38.2 -> 36.1.  The diagonal
+// block's and the FP64 sweeps round differently in the two forms and keep the grid
+// (eight models with the diagonal block 67.5 against 72.7 ms).
+bool Solver::passes_in_batch(const Level &Lv) const
+{
+    return in_batch && Lv.res_mode == 2 && prm.precision == 0 && prm.smoother == 1;
+}
+
 template <typename T>
 void Solver::smooth(int l, int sweeps)
 {
     Level &Lv = L[l];
     LevelView<T> V = view<T>(l, false);
     Vec4<T> &x = vx_of<T>(Lv, 0), &y = vx_of<T>(Lv, 1), &b = b_of<T>(Lv);
-    if (sweeps > 0 && Lv.res_mode && (prm.smoother == 0 || prm.smoother == 1)) {
+    const bool passes = passes_in_batch(Lv);
+    if (sweeps > 0 && Lv.res_mode && !passes && (prm.smoother == 0 || prm.smoother == 1)) {
         if (prm.smoother == 1) smooth_resident<T, true>(l, sweeps);
         else smooth_resident<T, false>(l, sweeps);
         return;
     }
-    if (sweeps <= 0 || use_fused(l) || Lv.res_mode) bc_set<T>(l, x, b);
+    if (sweeps <= 0 || use_fused(l) || (Lv.res_mode && !passes)) bc_set<T>(l, x, b);
     if (sweeps <= 0) return;
     // colour 0 reads velocities from x and writes y, colour 1 goes back; the
     // pressure is updated in place in x.c[0] (yy shares it)
@@ -1383,7 +1395,7 @@ void Solver::smooth(int l, int sweeps)
         }
         return;
     }
-    const bool follow = !Lv.res_mode && Lv.nbc > 0;
+    const bool follow = (!Lv.res_mode || passes) && Lv.nbc > 0;
     if (follow)
         pdl_launch(st, nblk(Lv.nbc), kThreads, k_bc_begin<T>, Lv.nbc, (const int *)Lv.bu, (const int *)Lv.bt,
                    (const float *)Lv.bk, (const int *)Lv.bnext, (const int *)Lv.follow_slot, x, yy, b,
@@ -1533,7 +1545,7 @@ void Solver::precondition()
 template <typename T>
 void Solver::capture_vcycle_graph()
 {
-    GraphSlot &g = (coarse_mode ? graphs_apx : graphs)[std::is_same<T, double>::value ? 1 : 0];
+    GraphSlot &g = vcycle_graph<T>();
     if (g.exec || !prm.use_graphs) return;
     long long before = g_launches;
     Capture capture(st);
@@ -1547,8 +1559,7 @@ void Solver::capture_vcycle_graph()
 template <typename T>
 void Solver::run_vcycle_graph()
 {
-    int key = std::is_same<T, double>::value ? 1 : 0;
-    GraphSlot &g = (coarse_mode ? graphs_apx : graphs)[key];
+    GraphSlot &g = vcycle_graph<T>();
     if (!prm.use_graphs) {
         vcycle<T>();
         P2_CUDA_TRY(cudaGetLastError());

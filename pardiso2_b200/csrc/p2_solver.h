@@ -176,6 +176,8 @@ class Solver {
     p2_tune_info autotune(int trial_iters);
     bool verbose = false;
 
+    bool in_batch = false;  // other solves run at the same time (p2_stokes_solve_batch)
+
     int dev;
     cudaStream_t st = nullptr;
     cudaEvent_t ev[8];
@@ -249,6 +251,12 @@ class Solver {
     void launch_restrict(int l, const Vec4<T> &r, const Vec4<T> &b, const Vec4<T> &x, const T *ws);
 
     template <typename T>
+    GraphSlot &vcycle_graph()
+    {
+        return (coarse_mode ? graphs_apx : graphs)[sizeof(T) / 8 + (in_batch ? 2 : 0)];
+    }
+    bool passes_in_batch(const Level &Lv) const;
+    template <typename T>
     void vcycle();
     template <typename T>
     void run_vcycle_graph();
@@ -272,10 +280,10 @@ class Solver {
 
     DeviceArena arena, grid_arena, marker_arena, move_arena, post_arena, heat_arena, heat_mk_arena;
     HeatState heat;
-    std::array<GraphSlot, 2> graphs;
+    std::array<GraphSlot, 4> graphs;  // float, double; the same in a batch
     // Coarsest LU + inverse on a second stream, overlapped with the first
     // lu_overlap_iters outer iterations, whose V-cycles smooth the coarsest level.
-    std::array<GraphSlot, 2> graphs_apx;
+    std::array<GraphSlot, 4> graphs_apx;
     cudaStream_t st_lu = nullptr;
     cudaEvent_t ev_lu = nullptr;
     bool lu_pending = false;
