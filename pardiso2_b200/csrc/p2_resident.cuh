@@ -16,7 +16,8 @@
 // the barrier, one round of loads from L2 and one cell's chain of about 600
 // instructions.  V-cycles: 33^3 0.260 -> 0.231 ms, 129^3 with doubling sweeps
 // 4.03 -> 3.26 ms, 257^3 11.76 -> 11.15 ms.  The grid form keeps every SM for its
-// launch: eight solves at once take 74.6 ms with it, 71.8 ms with clusters only.
+// launch, so concurrent solves take passes where those give the same bits
+// (Solver::passes_in_batch).
 #pragma once
 
 #include "p2_barrier.cuh"

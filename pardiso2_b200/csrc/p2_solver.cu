@@ -40,10 +40,12 @@ constexpr int kCoarseApxSweeps = 16;
 constexpr int kSweepChunk = 32;
 // Outer iterations that use the smoothed coarsest level: kOverlapScale *
 // nF / n0, fixed from the grid sizes so that the iterates do not depend on
-// timing (6 at 33^3, 0 from 65^3 on, all with nF = 3644).  The inverse
+// timing (6 at 33^3, 4 to 1 at 37^3 to 45^3, 0 from 49^3 on).  The inverse
 // fills the device, so running it beside the V-cycles gains little, and each
-// such iteration reduces the residual less: 33^3 8.3 ms without, 8.0 ms with 6, 9.0
-// ms with 16; 65^3 41.4 / 49.1 ms (two models) without, 45.9 / 52.5 ms with 5.
+// such iteration reduces the residual less.  Sums over six models to 1e-8 with
+// the rule / without, three sweep schedules: 33^3 mixed 45.6 to 47.6 / 48.5 to 52.4 ms,
+// FP64 53.2 to 57.4 / 56.0 to 61.2; 37^3, 41^3 and 45^3 2 to 7 % less in both
+// precisions.  16 at 33^3 cost 9.0 against 8.3 ms of one model, 5 at 65^3 45.9 against 41.4.
 // None on grids of one or two levels, where the coarsest level is too large a
 // part of the problem for smoothing to stand in for it.  The solve waits for the
 // inverse at that iteration if it is still running.
@@ -2146,8 +2148,8 @@ double Solver::debug_time_sweep(int l, int sweeps)
 
 // Average device time of one stage of the solve on the state left by the
 // last solve, each repetition timed alone after a 256 MB write that evicts
-// L2: 0 the V-cycle residual of `level` (its rows kernel chosen by variant:
-// 0 by grid size and precision, 1 k_rows, 2 k_rows_zm), 1 the level-0
+// L2: 0 the V-cycle residual of `level` (its rows kernel by variant: 0 and 1
+// k_rows, which solves use, 2 k_rows_zm), 1 the level-0
 // FP64 true residual with its float copy (same variants), 2 the restriction
 // of `level` to level + 1, 3 the prolongation of level + 1 to `level`, 4 the
 // level-0 FP64 operator q = A z (rows variants).

@@ -167,7 +167,7 @@ class Solver {
     double debug_time_smoother(int level, int passes);
     double debug_time_sweep(int level, int sweeps);
     double debug_time_stage(int stage, int level, int variant, int reps);
-    int dbg_rows_variant = 0;     // kernel of the operator rows (launch_rows), 0 = by grid size and precision
+    int dbg_rows_variant = 0;     // kernel of the operator rows (launch_rows): 0 and 1 k_rows, 2 k_rows_zm
     int dbg_forms = 0;            // resident sweeps as if the device placed no cluster (1), nor a cooperative grid (2)
     void drop_graphs_public() { drop_graphs(); }
     void debug_smooth(int level, int sweeps, const double *b, double *x);
