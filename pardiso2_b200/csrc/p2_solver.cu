@@ -955,11 +955,12 @@ void Solver::build_coarse_index()
     Ainv64 = (double *)arena.alloc(sizeof(double) * (size_t)gj.n * gj.n);
     Ainv32 = (float *)arena.alloc(sizeof(float) * (size_t)gj.n * gj.n);
     gj_work = (double *)arena.alloc(sizeof(double) * gj_work_doubles(gj.n));
-    d_row_scale = (double *)arena.alloc(sizeof(double) * nF);
     d_ipiv = (int *)arena.alloc(sizeof(int) * nF);
     d_info = (int *)arena.alloc(sizeof(int) * 4);
     probes = (double *)arena.alloc(sizeof(double) * (size_t)C.n * 4 * kProbes);
-    d_bw = (int *)arena.alloc(sizeof(int) * 2);
+    // the rows' scales and, after them, the band: cleared together
+    d_row_scale = (double *)arena.alloc(sizeof(double) * (nF + 1));
+    d_bw = (int *)(d_row_scale + nF);
     if (!h_bw) {
         int *p = nullptr;
         P2_CUDA_TRY(cudaMallocHost(&p, sizeof(int) * 2));
@@ -1035,7 +1036,9 @@ __global__ void k_probe_rows(LevelView<double> Lc, const double *probes, const i
         if (a != 0.0) {
             if (row > col) atomicMax(&bw[0], row - col);
             if (col > row) atomicMax(&bw[1], col - row);
-            if (comp) atomicMax(scale + row, (unsigned long long)__double_as_longlong(fabs(a)));  // orders as the values do
+            // a momentum row's largest velocity entry is its diagonal; the bits of a magnitude order as it does
+            if (c && row == col) scale[row] = (unsigned long long)__double_as_longlong(fabs(a));
+            else if (c == 0 && comp) atomicMax(scale + row, (unsigned long long)__double_as_longlong(fabs(a)));
         }
     }
 }
@@ -1050,10 +1053,9 @@ void Solver::coarse_setup(int way)
     int nl = (int)L.size();
     LevelView<double> Lc = view<double>(nl - 1, nl == 1);
     P2_CUDA_TRY(cudaMemsetAsync(A_c, 0, sizeof(double) * (size_t)nF * nF, st));
-    P2_CUDA_TRY(cudaMemsetAsync(d_bw, 0, sizeof(int) * 2, st));
+    P2_CUDA_TRY(cudaMemsetAsync(d_row_scale, 0, sizeof(double) * (nF + 1), st));
     dim3 grid(nblk(C.n), kProbes);
     k_probe_build<<<grid, kThreads, 0, st>>>(C.nx, C.ny, C.nz, d_colmap, d_crt, d_crk, probes); P2_COUNT_LAUNCH();
-    P2_CUDA_TRY(cudaMemsetAsync(d_row_scale, 0, sizeof(double) * nF, st));
     k_probe_rows<<<grid, kThreads, 0, st>>>(Lc, probes, d_colmap, A_c, nF, d_bw, (unsigned long long *)d_row_scale); P2_COUNT_LAUNCH();
     P2_CUDA_TRY(cudaGetLastError());
     // The inverse runs on its own stream; the solve goes on with a smoothed

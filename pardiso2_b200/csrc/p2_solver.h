@@ -323,7 +323,7 @@ class Solver {
     float *Ainv32 = nullptr;
     int *d_ipiv = nullptr, *d_info = nullptr;
     double *probes = nullptr;
-    int *d_bw = nullptr, *h_bw = nullptr;  // band of the coarsest operator (kl, ku)
+    int *d_bw = nullptr, *h_bw = nullptr;  // band of the coarsest operator (kl, ku), behind d_row_scale
     std::shared_ptr<int> h_bw_keep;
     double *cpart64 = nullptr;             // partial products of the coarsest solve
     float *cpart32 = nullptr;
