@@ -399,10 +399,12 @@ struct TransferView {
 };
 
 // Boundary rows that follow a regular unknown: row, resolved target and the
-// product of the chain's coefficients in the cycle's type.
+// product of the chain's coefficients; in the FP64 cycle the target's top bit is
+// set where no float holds the product (kd then).
 struct BcFollow {
     int n;
     const int *uc, *target;
-    const void *k;
+    const float *k;
+    const double *kd;
 };
 }  // namespace p2

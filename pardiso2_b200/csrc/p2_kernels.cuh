@@ -193,10 +193,12 @@ __global__ void k_bc_follow(BcFollow R, const T *c, Vec4<T> x)
     pdl_enter();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= R.n) return;
-    const int uc = __ldg(R.uc + q), t = __ldg(R.target + q);
+    const int uc = __ldg(R.uc + q), tk = __ldg(R.target + q), t = tk & 0x7fffffff;
+    T k = (T)__ldg(R.k + q);
+    if (sizeof(T) == 8 && tk < 0) k = (T)__ldg(R.kd + q);
     const T *s = (t & 3) == 0 ? x.c[0] : ((t & 3) == 1 ? x.c[1] : ((t & 3) == 2 ? x.c[2] : x.c[3]));
     T *d = (uc & 3) == 0 ? x.c[0] : ((uc & 3) == 1 ? x.c[1] : ((uc & 3) == 2 ? x.c[2] : x.c[3]));
-    d[uc >> 2] = __ldg(c + q) + __ldg((const T *)R.k + q) * s[t >> 2];
+    d[uc >> 2] = __ldg(c + q) + k * s[t >> 2];
 }
 // Start of a smoothing call: every boundary row of x (as k_bc_set_chain) and,
 // in the second velocity buffer y, the same values, which the rows without a

@@ -31,15 +31,15 @@ constexpr int kResCluster = 16;
 
 // Boundary rows for the resident sweeps: the rows' chains as for
 // k_bc_set_chain, and per colour and slot the rows that follow one of the
-// cell's unknowns: {unknown * 8 + face (0..5, 6 for the pressure), row} and the
-// product of the chain's coefficients in the cycle's type.
+// cell's unknowns: {unknown * 8 + face (0..5, 6 for the pressure), row, bits of the
+// product of the chain's coefficients}: a float's, or the two halves of a double
+// where no float holds it (the first entry then has its top bit set).
 struct ResidentBC {
     int nbc;
     const int *bu, *bt, *bnext;
     const float *bk;
     const int *ptr;
-    const int2 *dep;
-    const void *depk;
+    const int4 *dep;
     int cap;  // most entries of one block
 };
 
@@ -60,8 +60,9 @@ __host__ __device__ constexpr int res_values() { return kFull ? kBlkEntries : 7;
 // a row that follows an unknown of the block's cells: its constant part, coefficient, unknown and face
 template <typename T>
 struct ResDep {
-    T c, k;
-    int what;  // unknown * 8 + face
+    T c;
+    float k;
+    int what;  // as in ResidentBC::dep
 };
 constexpr size_t kResSmemMax = 227 * 1024 - 64;
 template <typename T, bool kFull>
@@ -161,9 +162,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_smooth_resident(LevelView<T>
         y.c[uc & 3][uc >> 2] = v;
     }
     for (int e = tid; e < n0 + n1; e += nt) {
-        const int at = e < n0 ? e0 + e : e1 + e - n0;
-        const int2 D = R.dep[at];
-        deps[e] = ResDep<T>{row_value(D.y, true), ((const T *)R.depk)[at], D.x};
+        const int4 D = R.dep[e < n0 ? e0 + e : e1 + e - n0];
+        deps[e] = ResDep<T>{row_value(D.y, true), D.x < 0 ? (float)__hiloint2double(D.w, D.z) : __int_as_float(D.z), D.x};
     }
     __syncthreads();  // the tables and entries
     if (!kFull && valid) {
@@ -252,12 +252,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_smooth_resident(LevelView<T>
             if (pown) o0[u] = p;
             for (int e = d0; e < d1; e++) {
                 const ResDep<T> D = deps[e];
-                const int face = D.what & 7, uc = D.what >> 3;
+                const int face = D.what & 7, uc = (D.what & 0x7fffffff) >> 3;
                 if (!mine && face != 6) continue;
+                T dk = (T)D.k;
+                if (sizeof(T) == 8 && D.what < 0) {
+                    const int4 X = R.dep[e < n0 ? e0 + e : e1 + e - n0];
+                    dk = (T)__hiloint2double(X.w, X.z);
+                }
                 const T v = face == 0 ? vn[0] : face == 1 ? vn[1] : face == 2 ? vn[2] : face == 3 ? vn[3]
                           : face == 4 ? vn[4] : face == 5 ? vn[5] : p;
                 T *o = (uc & 3) == 0 ? o0 : ((uc & 3) == 1 ? o1 : ((uc & 3) == 2 ? o2 : o3));
-                o[uc >> 2] = D.c + D.k * v;
+                o[uc >> 2] = D.c + dk * v;
             }
         }
         swap(i0, o0); swap(i1, o1); swap(i2, o2); swap(i3, o3);

@@ -12,9 +12,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <map>
 #include <memory>
 #include <string>
@@ -217,13 +219,6 @@ static V *upload(DeviceArena &A, const std::vector<V> &h)
     V *d = (V *)A.alloc(sizeof(V) * std::max<size_t>(h.size(), 1));
     if (!h.empty()) P2_CUDA_TRY(cudaMemcpy(d, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice));
     return d;
-}
-
-// Values in the V-cycle's type.
-void *Solver::upload_cycle(const std::vector<double> &v)
-{
-    if (prm.precision == 1) return upload(arena, v);
-    return upload(arena, std::vector<float>(v.begin(), v.end()));
 }
 
 static AxisMap upload_axis(DeviceArena &A, const HostAxis &h, bool restriction = false)
@@ -607,15 +602,17 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
         build_resident(Lv);
         if (!Lv.res_mode || (Lv.res_mode == 2 && prm.precision == 0)) {
             std::vector<int> slot(Lv.h_bu.size(), -1), uc, target;
-            std::vector<double> k;
+            std::vector<float> k;
+            std::vector<double> kd;
             for (size_t q = 0; q < Lv.h_bu.size(); q++) {
                 if (Lv.h_rt[q] < 0) continue;
                 slot[q] = (int)uc.size();
                 uc.push_back(Lv.h_bu[q]);
-                target.push_back(Lv.h_rt[q]);
-                k.push_back(Lv.h_rk[q]);
+                k.push_back((float)Lv.h_rk[q]);
+                kd.push_back(Lv.h_rk[q]);
+                target.push_back(Lv.h_rt[q] | (prm.precision == 1 && (double)k.back() != kd.back() ? INT_MIN : 0));
             }
-            Lv.follow = BcFollow{(int)uc.size(), upload(arena, uc), upload(arena, target), upload_cycle(k)};
+            Lv.follow = BcFollow{(int)uc.size(), upload(arena, uc), upload(arena, target), upload(arena, k), upload(arena, kd)};
             Lv.follow_slot = upload(arena, slot);
             Lv.follow_const = arena.alloc(sizeof(double) * std::max<size_t>(uc.size(), 1));
         }
@@ -710,24 +707,24 @@ bool Solver::build_resident_rows(Level &Lv)
     Lv.res_slots = per_block(Lv.res_blocks);
     // two passes over the rows: count per colour and slot, then place
     std::vector<int> ptr(2 * slots + 1, 0), at;
-    std::vector<int2> dep;
-    std::vector<double> depk;
+    std::vector<int4> dep;
     for (int pass = 0; pass < 2; pass++) {
         for (size_t q = 0; q < Lv.h_bu.size(); q++) {
             const int t = Lv.h_rt[q];
             if (t < 0) continue;
             const int c = t & 3, v = t >> 2;
+            const float rk = (float)Lv.h_rk[q];
+            const bool exact = (double)rk == Lv.h_rk[q];
+            int kbits[2] = {0, 0};
+            if (exact) std::memcpy(kbits, &rk, sizeof rk);
+            else std::memcpy(kbits, &Lv.h_rk[q], sizeof(double));
             const int j = v % Lv.ny, i = (v / Lv.ny) % Lv.nx, k = v / (Lv.nx * Lv.ny);
             auto follow = [&](int ci, int cj, int ck, int face) {
                 // a target that is no cell's unknown keeps its value through the sweeps
                 if (ci < 1 || cj < 1 || ck < 1 || ci >= Lv.nx || cj >= Lv.ny || ck >= Lv.nz) return;
                 const long slot = ((ci + cj + ck) & 1) * slots + ((long)(ck - 1) * (Lv.nx - 1) + (ci - 1)) * half + (cj - 1) / 2;
-                if (pass == 0) {
-                    ptr[slot + 1]++;
-                } else {
-                    depk[at[slot]] = Lv.h_rk[q];
-                    dep[at[slot]++] = make_int2(Lv.h_bu[q] * 8 + face, (int)q);
-                }
+                if (pass == 0) ptr[slot + 1]++;
+                else dep[at[slot]++] = make_int4((Lv.h_bu[q] * 8 + face) | (exact ? 0 : INT_MIN), (int)q, kbits[0], kbits[1]);
             };
             // the cells on both sides of a face (one of each colour), or the pressure's own cell
             if (c == 0) follow(i, j, k, 6);
@@ -739,7 +736,6 @@ bool Solver::build_resident_rows(Level &Lv)
             for (long e = 0; e < 2 * slots; e++) ptr[e + 1] += ptr[e];
             at.assign(ptr.begin(), ptr.end() - 1);
             dep.resize(ptr[2 * slots]);
-            depk.resize(ptr[2 * slots]);
         }
     }
     Lv.res_cap = 0;
@@ -753,7 +749,6 @@ bool Solver::build_resident_rows(Level &Lv)
     if (most > kResSmemMax) return false;
     Lv.res_ptr = upload(arena, ptr);
     Lv.res_dep = upload(arena, dep);
-    Lv.res_depk = upload_cycle(depk);
     return true;
 }
 
@@ -1332,7 +1327,7 @@ void Solver::smooth_resident(int l, int sweeps)
     Level &Lv = L[l];
     LevelView<T> V = view<T>(l, false);
     const int mx = Lv.tabstride;
-    const ResidentBC R{Lv.nbc, Lv.bu, Lv.bt, Lv.bnext, Lv.bk, Lv.res_ptr, Lv.res_dep, Lv.res_depk, Lv.res_cap};
+    const ResidentBC R{Lv.nbc, Lv.bu, Lv.bt, Lv.bnext, Lv.bk, Lv.res_ptr, Lv.res_dep, Lv.res_cap};
     const T *tab = std::is_same<T, double>::value ? (const T *)Lv.tabd : (const T *)Lv.tabf;
     ResidentKernel<T> kern;
     cudaLaunchConfig_t cfg;

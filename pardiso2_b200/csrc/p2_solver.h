@@ -53,8 +53,7 @@ struct Level {
     // resident sweeps (k_smooth_resident): 0 none, 1 one cluster, 2 cooperative grid
     int res_mode = 0, res_blocks = 0, res_slots = 0, res_cap = 0;
     int *res_ptr = nullptr;
-    int2 *res_dep = nullptr;
-    void *res_depk = nullptr;
+    int4 *res_dep = nullptr;
     // boundary rows between separate colour passes
     BcFollow follow{};
     int *follow_slot = nullptr;
@@ -232,7 +231,6 @@ class Solver {
     void smooth(int l, int sweeps);
     template <typename T, bool kFull>
     void smooth_resident(int l, int sweeps);
-    void *upload_cycle(const std::vector<double> &v);
     void build_resident(Level &Lv);
     bool build_resident_rows(Level &Lv);
     int sm_count = 0;
