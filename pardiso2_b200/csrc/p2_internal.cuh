@@ -53,6 +53,7 @@ constexpr int kGT = 64;  // tile edge and panel width
 struct GjPlan {
     int nF = 0, n = 0, nv = 0;  // unknowns, padded size, padded velocity part
     const int *perm = nullptr, *iperm = nullptr;
+    const double *scale = nullptr;  // of the continuity rows in A's order: their largest entry; 0 for momentum rows
     std::vector<int> tv, tq;
     bool lu_first = false;  // the pivoted band LU is the shorter way
 };

@@ -667,15 +667,13 @@ void band_lu_inverse(cudaStream_t st, double *A, int n, int kl, int ku, double *
 
 // Inverse of A (nF x nF, column-major) into X (n x n in the plan's order, see
 // p2_gj.cuh) and its float copy Xf (or null); d_flag is set when a pivot is not
-// positive or the check of the inverse fails (scale: of every row of A).  A is
-// only read.
-static void gj_issue(cudaStream_t st, const double *A, const double *scale, const GjPlan &P, double *X, float *Xf,
-                     double *work, int *d_flag)
+// positive or the check of the inverse fails.  A is only read.
+static void gj_issue(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag)
 {
     const int n = P.n, nt = n / kGT;
     double *Lb = work, *Ub = Lb + (size_t)kGT * n, *D = Ub + (size_t)kGT * n, *y = D + 4 * kGT * kGT, *v = y + n;
     P2_CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), st));
-    k_gj_gather<<<dim3(n, (n + 255) / 256), 256, 0, st>>>(n, P.nF, P.perm, A, scale, X, v); P2_COUNT_LAUNCH();
+    k_gj_gather<<<dim3(n, (n + 255) / 256), 256, 0, st>>>(n, P.nF, P.perm, A, P.scale, X, v); P2_COUNT_LAUNCH();
     k_gj_first<<<1, kGThreads, 0, st>>>(X, n, D, d_flag); P2_COUNT_LAUNCH();
     for (int p = 0; p < nt; p++) {
         const GjTiles T{P.tv[p], P.tq[p], P.nv / kGT};
@@ -695,8 +693,8 @@ size_t gj_work_doubles(int n) { return (size_t)2 * kGT * n + 4 * kGT * kGT + 2 *
 // gj_issue replayed as one graph.  The capture holds the plan and every buffer;
 // the caller drops it with them (a key of sizes and addresses would not do: a
 // freed buffer's address comes back).
-void gj_inverse(cudaStream_t st, const double *A, const double *scale, const GjPlan &P, double *X, float *Xf, double *work,
-                int *d_flag, LuGraph *cache)
+void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
+                LuGraph *cache)
 {
     // per-device attributes, set on the current device (host-side calls)
     P2_CUDA_TRY(cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
@@ -704,7 +702,7 @@ void gj_inverse(cudaStream_t st, const double *A, const double *scale, const GjP
     if (!cache->exec) {
         const long long before = g_launches;
         Capture capture(st);
-        gj_issue(st, A, scale, P, X, Xf, work, d_flag);
+        gj_issue(st, A, P, X, Xf, work, d_flag);
         cache->kernels = g_launches - before;
         g_launches = before;
         capture.instantiate(&cache->exec);

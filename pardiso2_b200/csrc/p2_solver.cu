@@ -55,7 +55,7 @@ constexpr double kOverlapScale = 60.0;
 constexpr int kOverlapMax = 16;
 void d2f(cudaStream_t st, size_t n, const double *a, float *b);
 size_t gj_work_doubles(int n);
-void gj_inverse(cudaStream_t st, const double *A, const double *scale, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
+void gj_inverse(cudaStream_t st, const double *A, const GjPlan &P, double *X, float *Xf, double *work, int *d_flag,
                 LuGraph *cache);
 void permute_inverse(cudaStream_t st, const GjPlan &P, const double *B, double *X);
 
@@ -932,6 +932,12 @@ void Solver::build_coarse_index()
                 if (lo[u] >= 0 && hi[u + corner] >= 0) band = std::max(band, hi[u + corner] - lo[u]);
         }
         gj.lu_first = gj_prefers_lu(nF, gj.nv, band);
+        std::vector<double> scale(nF, 0.0);
+        for (int q : part[1]) {
+            const int u = fre[q] >> 2, j = u % C.ny, i = (u / C.ny) % C.nx, k = u / plane_nodes;
+            scale[q] = 1.0 / std::min({C.g[0][i] - C.g[0][i - 1], C.g[1][j] - C.g[1][j - 1], C.g[2][k] - C.g[2][k - 1]});
+        }
+        gj.scale = upload(arena, scale);
         gj.perm = upload(arena, perm);
         gj.iperm = upload(arena, iperm);
         d_slots = upload(arena, list);
@@ -953,9 +959,7 @@ void Solver::build_coarse_index()
     d_ipiv = (int *)arena.alloc(sizeof(int) * nF);
     d_info = (int *)arena.alloc(sizeof(int) * 4);
     probes = (double *)arena.alloc(sizeof(double) * (size_t)C.n * 4 * kProbes);
-    // the rows' scales and, after them, the band: cleared together
-    d_row_scale = (double *)arena.alloc(sizeof(double) * (nF + 1));
-    d_bw = (int *)(d_row_scale + nF);
+    d_bw = (int *)arena.alloc(sizeof(int) * 2);
     if (!h_bw) {
         int *p = nullptr;
         P2_CUDA_TRY(cudaMallocHost(&p, sizeof(int) * 2));
@@ -974,7 +978,7 @@ void Solver::build_coarse_index()
 // within two nodes.  All kProbes probes are built and applied in one launch
 // each (blockIdx.y = probe); the row kernel also records the band of the
 // operator in the free-unknown ordering (bw[0] = max row - col, bw[1] = max
-// col - row over the non-zeros) and every row's scale, its largest velocity entry.
+// col - row over the non-zeros).
 
 __global__ void k_probe_build(int nx, int ny, int nz, const int *colmap, const int *rt, const float *rk,
                               double *probes)
@@ -1001,7 +1005,7 @@ __global__ void k_probe_build(int nx, int ny, int nz, const int *colmap, const i
 }
 
 __global__ void k_probe_rows(LevelView<double> Lc, const double *probes, const int *colmap, double *A, int nF,
-                             int *bw, unsigned long long *scale)
+                             int *bw)
 {
     int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= Lc.n) return;
@@ -1031,9 +1035,6 @@ __global__ void k_probe_rows(LevelView<double> Lc, const double *probes, const i
         if (a != 0.0) {
             if (row > col) atomicMax(&bw[0], row - col);
             if (col > row) atomicMax(&bw[1], col - row);
-            // a momentum row's largest velocity entry is its diagonal; the bits of a magnitude order as it does
-            if (c && row == col) scale[row] = (unsigned long long)__double_as_longlong(fabs(a));
-            else if (c == 0 && comp) atomicMax(scale + row, (unsigned long long)__double_as_longlong(fabs(a)));
         }
     }
 }
@@ -1048,10 +1049,10 @@ void Solver::coarse_setup(int way)
     int nl = (int)L.size();
     LevelView<double> Lc = view<double>(nl - 1, nl == 1);
     P2_CUDA_TRY(cudaMemsetAsync(A_c, 0, sizeof(double) * (size_t)nF * nF, st));
-    P2_CUDA_TRY(cudaMemsetAsync(d_row_scale, 0, sizeof(double) * (nF + 1), st));
+    P2_CUDA_TRY(cudaMemsetAsync(d_bw, 0, sizeof(int) * 2, st));
     dim3 grid(nblk(C.n), kProbes);
     k_probe_build<<<grid, kThreads, 0, st>>>(C.nx, C.ny, C.nz, d_colmap, d_crt, d_crk, probes); P2_COUNT_LAUNCH();
-    k_probe_rows<<<grid, kThreads, 0, st>>>(Lc, probes, d_colmap, A_c, nF, d_bw, (unsigned long long *)d_row_scale); P2_COUNT_LAUNCH();
+    k_probe_rows<<<grid, kThreads, 0, st>>>(Lc, probes, d_colmap, A_c, nF, d_bw); P2_COUNT_LAUNCH();
     P2_CUDA_TRY(cudaGetLastError());
     // The inverse runs on its own stream; the solve goes on with a smoothed
     // coarsest level for lu_overlap_iters outer iterations.
@@ -1061,7 +1062,7 @@ void Solver::coarse_setup(int way)
     if (lu_pivoted) {
         invert_pivoted();
     } else {
-        gj_inverse(st_lu, A_c, d_row_scale, gj, Ainv64, prm.precision == 0 ? Ainv32 : nullptr, gj_work, d_info, &lu_graph);
+        gj_inverse(st_lu, A_c, gj, Ainv64, prm.precision == 0 ? Ainv32 : nullptr, gj_work, d_info, &lu_graph);
         P2_CUDA_TRY(cudaEventRecord(ev_lu, st_lu));
     }
     lu_pending = true;

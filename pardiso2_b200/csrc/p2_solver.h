@@ -312,7 +312,7 @@ class Solver {
     int *d_colmap = nullptr, *d_crt = nullptr;
     GjPlan gj;
     int *d_slots = nullptr, *d_slot_of = nullptr;  // unknown of each slot of the inverse (-1 padding), and back
-    double *gj_work = nullptr, *d_row_scale = nullptr;
+    double *gj_work = nullptr;
     LuGraph lu_graph_pivoted;
     void invert_pivoted();
     bool lu_pivoted = false;  // the inverse in flight is the pivoted LU's
@@ -321,7 +321,7 @@ class Solver {
     float *Ainv32 = nullptr;
     int *d_ipiv = nullptr, *d_info = nullptr;
     double *probes = nullptr;
-    int *d_bw = nullptr, *h_bw = nullptr;  // band of the coarsest operator (kl, ku), behind d_row_scale
+    int *d_bw = nullptr, *h_bw = nullptr;  // band of the coarsest operator (kl, ku)
     std::shared_ptr<int> h_bw_keep;
     double *cpart64 = nullptr;             // partial products of the coarsest solve
     float *cpart32 = nullptr;
