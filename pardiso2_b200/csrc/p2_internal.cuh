@@ -400,8 +400,8 @@ struct TransferView {
 };
 
 // Boundary rows that follow a regular unknown: row, resolved target and the
-// product of the chain's coefficients; in the FP64 cycle the target's top bit is
-// set where no float holds the product (kd then).
+// product of the chain's coefficients; kd: the products of the FP64 cycle, on
+// levels where no float holds one of them, else null.
 struct BcFollow {
     int n;
     const int *uc, *target;

@@ -187,15 +187,14 @@ __global__ void k_bc_set_chain(int nbc, const int *bu, const int *bt, const floa
 // regular target, by their resolved target and the constant part that
 // k_bc_begin left for them, x = c + k x_target.  Two dependent loads instead of
 // the walk along the chain: V-cycle of 65^3 0.491 -> 0.444 ms, of 257^3 10.64 -> 10.21 ms.
-template <typename T>
+template <typename T, bool kDouble>
 __global__ void k_bc_follow(BcFollow R, const T *c, Vec4<T> x)
 {
     pdl_enter();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= R.n) return;
-    const int uc = __ldg(R.uc + q), tk = __ldg(R.target + q), t = tk & 0x7fffffff;
-    T k = (T)__ldg(R.k + q);
-    if (sizeof(T) == 8 && tk < 0) k = (T)__ldg(R.kd + q);
+    const int uc = __ldg(R.uc + q), t = __ldg(R.target + q);
+    const T k = kDouble ? (T)__ldg(R.kd + q) : (T)__ldg(R.k + q);
     const T *s = (t & 3) == 0 ? x.c[0] : ((t & 3) == 1 ? x.c[1] : ((t & 3) == 2 ? x.c[2] : x.c[3]));
     T *d = (uc & 3) == 0 ? x.c[0] : ((uc & 3) == 1 ? x.c[1] : ((uc & 3) == 2 ? x.c[2] : x.c[3]));
     d[uc >> 2] = __ldg(c + q) + k * s[t >> 2];

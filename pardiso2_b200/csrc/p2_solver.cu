@@ -604,15 +604,18 @@ void Solver::set_bc(const int *bondm, long bondm_len, const float *bondv1, const
             std::vector<int> slot(Lv.h_bu.size(), -1), uc, target;
             std::vector<float> k;
             std::vector<double> kd;
+            bool inexact = false;
             for (size_t q = 0; q < Lv.h_bu.size(); q++) {
                 if (Lv.h_rt[q] < 0) continue;
                 slot[q] = (int)uc.size();
                 uc.push_back(Lv.h_bu[q]);
                 k.push_back((float)Lv.h_rk[q]);
                 kd.push_back(Lv.h_rk[q]);
-                target.push_back(Lv.h_rt[q] | (prm.precision == 1 && (double)k.back() != kd.back() ? INT_MIN : 0));
+                target.push_back(Lv.h_rt[q]);
+                inexact = inexact || (double)k.back() != kd.back();
             }
-            Lv.follow = BcFollow{(int)uc.size(), upload(arena, uc), upload(arena, target), upload(arena, k), upload(arena, kd)};
+            Lv.follow = BcFollow{(int)uc.size(), upload(arena, uc), upload(arena, target), upload(arena, k),
+                                 inexact && prm.precision == 1 ? upload(arena, kd) : nullptr};
             Lv.follow_slot = upload(arena, slot);
             Lv.follow_const = arena.alloc(sizeof(double) * std::max<size_t>(uc.size(), 1));
         }
@@ -1406,7 +1409,8 @@ void Solver::smooth(int l, int sweeps)
             smoother_pass<T>(l, V, x.c[0], vin, vout, b, col);
             if (!follow) bc_set<T>(l, vout, b);
             else if (Lv.follow.n > 0)
-                pdl_launch(st, nblk(Lv.follow.n), kThreads, k_bc_follow<T>, Lv.follow, (const T *)Lv.follow_const, vout);
+                pdl_launch(st, nblk(Lv.follow.n), kThreads, Lv.follow.kd ? k_bc_follow<T, true> : k_bc_follow<T, false>,
+                           Lv.follow, (const T *)Lv.follow_const, vout);
         }
     }
 }
